@@ -175,11 +175,11 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 if (mf[k] != 0) {
-                    unsigned long long* a = G.acc + 4ull * node_index(P, x, y, rb[2] + 2 * half + k);
-                    atomicAdd(a + 0, (unsigned long long)mf[k]);
-                    atomicAdd(a + 1, to_fixed(gx[k], P.mom_scale));
-                    atomicAdd(a + 2, to_fixed(gy[k], P.mom_scale));
-                    atomicAdd(a + 3, to_fixed(gz[k], P.mom_scale));
+                    unsigned long long* a = acc_node(G, node_index(P, x, y, rb[2] + 2 * half + k));
+                    atomicAdd(a, (unsigned long long)mf[k]);
+                    atomicAdd(a + kAccX, to_fixed(gx[k], P.mom_scale));
+                    atomicAdd(a + kAccY, to_fixed(gy[k], P.mom_scale));
+                    atomicAdd(a + kAccZ, to_fixed(gz[k], P.mom_scale));
                 }
             }
         }
@@ -301,11 +301,11 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
         const int bx = t % kP2GTileBx, by = (t / kP2GTileBx) & 1, bz = t / (2 * kP2GTileBx);
         if (org[0] + bx >= P.nb[0]) continue;  // past the padded grid: nothing was added there
         const uint32_t gblk = (uint32_t)(((org[2] + bz) * P.nb[1] + org[1] + by) * P.nb[0] + org[0] + bx);
-        unsigned long long* a = G.acc + 4ull * ((gblk << 6) | (uint32_t)(i & 63));
+        unsigned long long* a = acc_node(G, (gblk << 6) | (uint32_t)(i & 63));
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const unsigned long long v = tacc[c * kP2GTileNodes + i];
-            if (v != 0ull) atomicAdd(a + c, v);
+            if (v != 0ull) atomicAdd(a + c * kAccX, v);
         }
     }
 }
@@ -326,23 +326,22 @@ __global__ void __launch_bounds__(256) k_normalize(KParams P, GArrays G, DevStat
     float vmax = 0.0f;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
         uint32_t node = ((uint32_t)G.active[i >> 6] << 6) | (uint32_t)(i & 63);
-        longlong2* a2 = reinterpret_cast<longlong2*>(G.acc + 4ull * node);
-        longlong2 a = a2[0], b = a2[1];
+        long long* a = reinterpret_cast<long long*>(acc_node(G, node));
+        const long long am = a[0], ax = a[kAccX], ay = a[kAccY], az = a[kAccZ];
         float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a.x > 0) {
+        if (am > 0) {
             ++cnt;
-            float m = __ll2float_rn(a.x) * P.inv_mass_scale;
+            float m = __ll2float_rn(am) * P.inv_mass_scale;
             float inv = 1.0f / m;
-            out = make_float4(__ll2float_rn(a.y) * P.inv_mom_scale * inv, __ll2float_rn(b.x) * P.inv_mom_scale * inv,
-                              __ll2float_rn(b.y) * P.inv_mom_scale * inv, m);
+            out = make_float4(__ll2float_rn(ax) * P.inv_mom_scale * inv, __ll2float_rn(ay) * P.inv_mom_scale * inv,
+                              __ll2float_rn(az) * P.inv_mom_scale * inv, m);
             vmax = fmaxf(vmax, out.x * out.x + out.y * out.y + out.z * out.z);
         }
         const long long lim = 1ll << 61;
-        ovf |= (a.x > lim) | (a.y > lim) | (a.y < -lim) | (b.x > lim) | (b.x < -lim) | (b.y > lim) | (b.y < -lim);
+        ovf |= (am > lim) | (ax > lim) | (ax < -lim) | (ay > lim) | (ay < -lim) | (az > lim) | (az < -lim);
         G.vel[node] = out;
-        a2[0] = make_longlong2(0, 0);
-        a2[1] = make_longlong2(0, 0);
-        sm_ += a.x; sx += a.y; sy += b.x; sz += b.y;
+        a[0] = a[kAccX] = a[kAccY] = a[kAccZ] = 0;
+        sm_ += am; sx += ax; sy += ay; sz += az;
     }
     if (P.vmax2) warp_max_atomic(P.vmax2 + 0, vmax);
 #pragma unroll
@@ -552,10 +551,10 @@ __global__ void k_force_fp64(KParams P, PArrays cur, GArrays G, float dt_force, 
                     const float g[3] = {dw[0][ox] * w[1][oy] * w[2][oz], w[0][ox] * dw[1][oy] * w[2][oz],
                                         w[0][ox] * w[1][oy] * dw[2][oz]};
                     if (g[0] == 0.0f && g[1] == 0.0f && g[2] == 0.0f) continue;
-                    unsigned long long* a = G.acc + 4ull * node_index(P, base[0] + ox, base[1] + oy, base[2] + oz);
+                    unsigned long long* a = acc_node(G, node_index(P, base[0] + ox, base[1] + oy, base[2] + oz));
                     for (int c = 0; c < 3; ++c) {
                         const float fc = S[3 * c] * g[0] + S[3 * c + 1] * g[1] + S[3 * c + 2] * g[2];
-                        atomicAdd(a + 1 + c, to_fixed(fc, P.mom_scale));
+                        atomicAdd(a + (1 + c) * kAccX, to_fixed(fc, P.mom_scale));
                     }
                 }
         atomicAdd(&st->fallbacks, 1ull);
@@ -708,10 +707,10 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
         for (int k = 0; k < 2; ++k) {
             const float gx = h ? fx[2 + k] : fx[k], gy = h ? fy[2 + k] : fy[k], gz = h ? fz[2 + k] : fz[k];
             if (gx != 0.0f || gy != 0.0f || gz != 0.0f) {
-                unsigned long long* a = G.acc + 4ull * node_index(P, x, y, rb[2] + 2 * h + k);
-                atomicAdd(a + 1, to_fixed(gx, P.mom_scale));
-                atomicAdd(a + 2, to_fixed(gy, P.mom_scale));
-                atomicAdd(a + 3, to_fixed(gz, P.mom_scale));
+                unsigned long long* a = acc_node(G, node_index(P, x, y, rb[2] + 2 * h + k));
+                atomicAdd(a + kAccX, to_fixed(gx, P.mom_scale));
+                atomicAdd(a + kAccY, to_fixed(gy, P.mom_scale));
+                atomicAdd(a + kAccZ, to_fixed(gz, P.mom_scale));
             }
         }
 #pragma unroll
@@ -766,16 +765,16 @@ __global__ void k_grid(KParams P, GArrays G, float dt_force, int write_force, do
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
         const uint32_t blk = (uint32_t)G.active[i >> 6];
         const uint32_t node = (blk << 6) | (uint32_t)(i & 63);
-        longlong2* a2 = reinterpret_cast<longlong2*>(G.acc + 4ull * node);
-        longlong2 a = a2[0], b = a2[1];
+        long long* a = reinterpret_cast<long long*>(acc_node(G, node));
+        const long long ax = a[kAccX], ay = a[kAccY], az = a[kAccZ];
         float4 v4 = G.vel[node];
         float4 bf = make_float4(0.f, 0.f, 0.f, 0.f);
         const float m = v4.w;
         if (m > 0.0f) {
             const float inv = P.inv_mom_scale / m;
-            float vx = v4.x + __ll2float_rn(a.y) * inv + dt_force * P.gravity[0];
-            float vy = v4.y + __ll2float_rn(b.x) * inv + dt_force * P.gravity[1];
-            float vz = v4.z + __ll2float_rn(b.y) * inv + dt_force * P.gravity[2];
+            float vx = v4.x + __ll2float_rn(ax) * inv + dt_force * P.gravity[0];
+            float vy = v4.y + __ll2float_rn(ay) * inv + dt_force * P.gravity[1];
+            float vz = v4.z + __ll2float_rn(az) * inv + dt_force * P.gravity[2];
             vmax = fmaxf(vmax, vx * vx + vy * vy + vz * vz);
             bf = make_float4(vx, vy, vz, 0.f);
             // node position (unpadded coordinates)
@@ -813,16 +812,15 @@ __global__ void k_grid(KParams P, GArrays G, float dt_force, int write_force, do
                 long ng = (long)P.res[0] * P.res[1] * P.res[2];
                 long idx = ((long)iz * P.res[1] + iy) * P.res[0] + ix;
                 double s = (double)P.inv_mom_scale / (double)dt_force;
-                force_out[idx] = (double)a.y * s;
-                force_out[ng + idx] = (double)b.x * s;
-                force_out[2 * ng + idx] = (double)b.y * s;
+                force_out[idx] = (double)ax * s;
+                force_out[ng + idx] = (double)ay * s;
+                force_out[2 * ng + idx] = (double)az * s;
             }
             continue;  // force stage: leave velocities and accumulators untouched
         }
         G.vel[node] = v4;
         G.vbf[node] = bf;
-        a2[0] = make_longlong2(0, 0);
-        a2[1] = make_longlong2(0, 0);
+        a[kAccX] = a[kAccY] = a[kAccZ] = 0;  // the mass is zero since the normalisation
         if ((i & 63) == 0) G.flag[blk] = 0u;
     }
     if (P.vmax2) warp_max_atomic(P.vmax2 + 1, vmax);
@@ -931,9 +929,8 @@ __global__ void k_grid_clear(GArrays G) {
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
         const uint32_t blk = (uint32_t)G.active[i >> 6];
         const uint32_t node = (blk << 6) | (uint32_t)(i & 63);
-        longlong2* a2 = reinterpret_cast<longlong2*>(G.acc + 4ull * node);
-        a2[0] = make_longlong2(0, 0);
-        a2[1] = make_longlong2(0, 0);
+        unsigned long long* a = acc_node(G, node);
+        a[0] = a[kAccX] = a[kAccY] = a[kAccZ] = 0ull;
         if ((i & 63) == 0) G.flag[blk] = 0u;
     }
 }
