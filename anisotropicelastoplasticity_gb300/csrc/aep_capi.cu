@@ -333,13 +333,15 @@ aep_status ensure_capacity(aep_solver* s, int64_t n, int64_t keep = 0) {
 // written by the conversion kernels directly over the host link), device and
 // managed memory; nullptr for pageable host memory, which goes through the
 // staging buffer.
-const void* device_alias(const void* p) {
+const void* device_alias(const void* p, bool* on_device = nullptr) {
+    if (on_device) *on_device = false;
     if (!p) return nullptr;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
+    if (on_device) *on_device = a.type == cudaMemoryTypeDevice;
     if (a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged) return a.devicePointer;
     if (a.type == cudaMemoryTypeDevice) return p;
     return nullptr;
@@ -347,9 +349,11 @@ const void* device_alias(const void* p) {
 
 // A device pointer with the caller's `bytes` at `p`: the alias, or a copy in the
 // staging buffer at `off` doubles
-const void* device_source(aep_solver* s, const void* p, size_t bytes, size_t off, cudaError_t* err) {
-    const void* a = device_alias(p);
+const void* device_source(aep_solver* s, const void* p, size_t bytes, size_t off, cudaError_t* err,
+                          bool* on_device = nullptr) {
+    const void* a = device_alias(p, on_device);
     if (a) return a;
+    if (on_device) *on_device = true;
     double* st = s->staging + off;
     *err = cudaMemcpyAsync(st, p, bytes, cudaMemcpyHostToDevice, s->stream);
     return st;
@@ -618,14 +622,7 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
         s->prev_sorted = false;
         s->cur = 0;
     }
-    const int32_t* map = nullptr;
-    if (keep_order) {
-        launch_inverse_ids((int)s->n, s->P[s->cur].id, s->perm, s->stream);  // over every item: ids 0..n-1 first
-        CKLAUNCH();
-        map = s->perm;
-    } else {
-        s->n = n;
-    }
+    if (!keep_order) s->n = n;
     s->np = n;
     PArrays& P = s->P[s->cur];
     // Arrays in page-locked host or device memory are read by the conversion
@@ -633,9 +630,13 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
     // Fe 15n, Fp 24n, m 33n, vol 34n, plastic 35n, material bytes at 36n.
     const size_t N = (size_t)n;
     cudaError_t e = cudaSuccess;
+    bool all_on_device = true;
     auto dsrc = [&](const void* p, size_t bytes, size_t off) -> const void* {
         if (!p || e != cudaSuccess) return nullptr;
-        return device_source(s, p, bytes, off, &e);
+        bool on_device = false;
+        const void* d = device_source(s, p, bytes, off, &e, &on_device);
+        all_on_device &= on_device;
+        return d;
     };
     UploadSrc src{static_cast<const double*>(dsrc(x, sizeof(double) * 3 * N, 0)),
                   static_cast<const double*>(dsrc(v, sizeof(double) * 3 * N, 3 * N)),
@@ -650,7 +651,18 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
     // the whole upload and its validation (bad masses, unknown tags, largest mass)
     // in one launch, read back with the final synchronisation
     CK(cudaMemsetAsync(s->check, 0, 2 * sizeof(unsigned long long), s->stream));
-    launch_upload_particles((int)n, src, P, map, s->prm.track_plastic_F, s->check, s->stream);
+    if (keep_order && all_on_device) {
+        launch_upload_slots((int)s->n, (int)n, src, P, s->prm.track_plastic_F, s->check, s->stream);
+    } else {
+        // host memory is read in its own order, whole lines over the link
+        const int32_t* map = nullptr;
+        if (keep_order) {
+            launch_inverse_ids((int)s->n, P.id, s->perm, s->stream);  // over every item: ids 0..n-1 first
+            CKLAUNCH();
+            map = s->perm;
+        }
+        launch_upload_particles((int)n, src, P, map, s->prm.track_plastic_F, s->check, s->stream);
+    }
     CKLAUNCH();
     unsigned long long* chk = s->check_host;
     CK(cudaMemcpyAsync(chk, s->check, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s->stream));
@@ -1377,7 +1389,8 @@ aep_status aep_get_particles(aep_solver* s, int64_t n, double* x, double* v, dou
     const int64_t np = s->np;
     const size_t N = (size_t)np;
     if ((st = prepare_download(s))) return st;
-    // one conversion launch for all requested fields: straight into page-locked or
+    // one conversion launch for the requested fields (matrices into device memory in their
+    // own): straight into page-locked or
     // device destinations, through staging (doubles: x 0, v 3N, B 6N, Fe 15N,
     // Fp 24N, vol 33N, plastic 34N) and one copy each for pageable ones
     double* const req[7] = {x, v, B, Fe, Fp, vol, plastic};
@@ -1385,14 +1398,22 @@ aep_status aep_get_particles(aep_solver* s, int64_t n, double* x, double* v, dou
     double* dev[7] = {};
     for (int f = 0; f < 7; ++f)
         if (req[f]) {
-            double* a = static_cast<double*>(const_cast<void*>(device_alias(req[f])));
+            bool on_device = false;
+            double* a = static_cast<double*>(const_cast<void*>(device_alias(req[f], &on_device)));
             dev[f] = a ? a : s->staging + off[f] * N;
+            if ((f == 3 || f == 4) && (on_device || !a)) {  // matrices in device memory leave from the slots' order
+                launch_download_F_slots((int)s->n, (int)np, dev[f], f == 3 ? P.F : P.Fp, P.id, s->stream);
+                CKLAUNCH();
+                if (!a)
+                    CK(cudaMemcpyAsync(req[f], dev[f], sizeof(double) * cnt[f] * N, cudaMemcpyDeviceToHost, s->stream));
+                dev[f] = nullptr;
+            }
         }
     DownloadDst dst{dev[0], dev[1], dev[2], dev[3], dev[4], dev[5], dev[6]};
     launch_download_particles((int)np, dst, P, s->inv, s->stream);
     CKLAUNCH();
     for (int f = 0; f < 7; ++f)
-        if (req[f] && dev[f] == s->staging + off[f] * N)
+        if (dev[f] && dev[f] == s->staging + off[f] * N)
             CK(cudaMemcpyAsync(req[f], dev[f], sizeof(double) * cnt[f] * N, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return AEP_OK;
