@@ -68,6 +68,7 @@ struct aep_solver {
     uint32_t* order_mem = nullptr;  // one allocation for the arrays below
     uint32_t* mk = nullptr;
     int32_t* mj = nullptr;
+    uint32_t* mprev = nullptr;
     uint32_t* mkeys = nullptr;
     int32_t* mslot = nullptr;
     int32_t* mpos = nullptr;
@@ -268,7 +269,7 @@ void free_particles(aep_solver* s) {
     s->iota = s->perm = nullptr;
     s->sort_tmp = nullptr;
     s->staging = nullptr;
-    s->order_mem = s->mk = s->mkeys = s->order_scratch = nullptr;
+    s->order_mem = s->mk = s->mprev = s->mkeys = s->order_scratch = nullptr;
     s->mj = s->mslot = s->mpos = nullptr;
     s->prev_sorted = false;
     s->cap = 0;
@@ -309,13 +310,14 @@ aep_status ensure_capacity(aep_solver* s, int64_t n, int64_t keep = 0) {
     // mover list and sorted mover keys (n / 4 + 1 each: more movers take the full sort)
     // and the ordering scratch
     const size_t mcap = (size_t)n / 4 + 1;
-    CK(cudaMalloc(&s->order_mem, sizeof(uint32_t) * (5 * mcap + order_scratch_words((int)n))));
+    CK(cudaMalloc(&s->order_mem, sizeof(uint32_t) * (6 * mcap + order_scratch_words((int)n))));
     s->mk = s->order_mem;
     s->mj = reinterpret_cast<int32_t*>(s->order_mem + mcap);
     s->mkeys = s->order_mem + 2 * mcap;
     s->mslot = reinterpret_cast<int32_t*>(s->order_mem + 3 * mcap);
     s->mpos = reinterpret_cast<int32_t*>(s->order_mem + 4 * mcap);
-    s->order_scratch = s->order_mem + 5 * mcap;
+    s->mprev = s->order_mem + 5 * mcap;
+    s->order_scratch = s->order_mem + 6 * mcap;
     if (!s->check_host) CK(cudaMallocHost(&s->check_host, 2 * sizeof(unsigned long long)));
     s->prev_sorted = false;
     s->staging_bytes = sizeof(double) * 37 * (size_t)n;  // every field of one particle set at once
@@ -431,7 +433,7 @@ inline void mark(aep_solver* s, int boundary) {
 // aep_sort.cu), or a full radix sort when there are no sorted keys yet.
 cudaError_t order_particles(aep_solver* s) {
     const int n = (int)s->n;
-    if (!s->prm.full_sort && s->prev_sorted && n >= 4096) {
+    if (!s->prm.full_sort && s->prev_sorted) {
         if (!s->order_graph || s->order_graph_n != n) {
             order_graph_destroy(s->order_graph);
             s->order_graph = nullptr;
@@ -439,7 +441,7 @@ cudaError_t order_particles(aep_solver* s) {
                 cudaError_t e = cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking);
                 if (e != cudaSuccess) return e;
             }
-            OrderBuffers b{s->keys, s->keys_sorted, s->perm, s->iota, s->mk, s->mj, s->mkeys, s->mslot, s->mpos,
+            OrderBuffers b{s->keys, s->keys_sorted, s->perm, s->iota, s->mk, s->mj, s->mprev, s->mkeys, s->mslot, s->mpos,
                            s->order_scratch, s->sort_tmp, s->sort_bytes, n, n / 4, s->key_bits, s->dstats};
             cudaError_t e = order_graph_build(&s->order_graph, s->capture_stream, b);
             if (e != cudaSuccess) return e;
@@ -472,7 +474,7 @@ aep_status run_p2g(aep_solver* s) {
     // reorder_interval: the steps between two orderings keep the particles in their
     // slots (identity permutation) with the keys G2P wrote for the current positions
     const int interval = std::max(1, (int)s->prm.reorder_interval);
-    if (s->prev_sorted && !s->prm.full_sort && s->n >= 4096 && s->since_order + 1 < interval) {
+    if (s->prev_sorted && !s->prm.full_sort && s->since_order + 1 < interval) {
         ++s->since_order;
         s->step_keys = s->keys;
         s->step_perm = s->iota;

@@ -75,6 +75,7 @@ struct OrderBuffers {
     const int32_t* iota;
     uint32_t* mk;          // mover list: keys and slots (cap entries)
     int32_t* mj;
+    uint32_t* mprev;       // and their previous keys
     uint32_t* mkeys;       // movers sorted by (key, slot): keys, slots, final positions
     int32_t* mslot;
     int32_t* mpos;

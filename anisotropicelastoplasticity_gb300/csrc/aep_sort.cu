@@ -36,28 +36,31 @@ namespace aep {
 // ===================================================================================
 // Stable LSD radix sort of (uint32 key, int32 value) pairs on the low key_bits bits.
 // The bits are cut into P = ceil(key_bits / 8) digits of R = ceil(key_bits / P) <= 8
-// bits.  Each pass is three kernels over tiles of kRsTile pairs:
+// bits.  Each pass is three kernels over tiles of kRsThreads x Rounds pairs:
 //   k_rs_hist     per tile, the count of every digit value -> hist[digit][tile]
 //   k_rs_scan     per digit (one block each): exclusive scan of its row over the
 //                 tiles in place, and the digit's total
-//   k_rs_scatter  per tile: the digits' bases (exclusive scan of the totals) plus
-//                 the row offsets give each digit's first output slot for the tile;
-//                 the tile is read in rounds of one pair per thread in input order,
-//                 and a pair's rank among the tile's equal digits comes from
-//                 __match_any_sync inside its warp, the counts of the warps before
-//                 it in the round and the running count of earlier rounds, so equal
-//                 digits keep their input order (the sort is stable).
+//   k_rs_scatter  per tile: each warp ranks its consecutive pairs round by round
+//                 (__match_any_sync inside the warp, the warp's running count of the
+//                 digit), the warps' counts and the digits' are scanned once, the tile is
+//                 sorted into shared memory and written out digit by digit: runs of
+//                 neighbouring output slots, equal digits in input order (stable)
 // Passes alternate between the output arrays and a scratch copy, arranged so that
 // the last pass writes the output.  Traffic per pass: keys and values read twice
 // and written once.
+// A tile is kRsThreads x Rounds pairs: 4 rounds (1,024 pairs) below kRsLarge pairs, 16
+// (4,096) from there on.  A tile's rounds run one after another, so a sort that leaves SMs
+// idle is faster with more, shorter tiles; a large one with fewer tile counts to scan.
+// Measured per sort, 4 against 16 rounds: 43 / 66 us for 131,072 pairs, 63 / 66 us for
+// 524,288, 140 / 152 us for 2,097,152, 422 / 403 us for 8,388,608 (90, 90, 184 and 599 us
+// with 16 rounds ranked with three block barriers each and written out unsorted).
 constexpr int kRsThreads = 256;
-constexpr int kRsRounds = 16;
-constexpr int kRsTile = kRsThreads * kRsRounds;  // 4096 pairs per tile
+constexpr int kRsLarge = 1 << 22;
 constexpr int kRsBins = 256;
 constexpr int kRsWarps = kRsThreads / 32;
 
 struct RsPlan {
-    int passes, radix, tiles;
+    int passes, radix, rounds, tiles;
 };
 
 RsPlan rs_plan(int n, int key_bits) {
@@ -65,17 +68,20 @@ RsPlan rs_plan(int n, int key_bits) {
     key_bits = std::max(1, std::min(32, key_bits));
     p.passes = (key_bits + 7) / 8;
     p.radix = (key_bits + p.passes - 1) / p.passes;
-    p.tiles = std::max(1, (n + kRsTile - 1) / kRsTile);
+    p.rounds = n < kRsLarge ? 4 : 16;
+    const int tile = kRsThreads * p.rounds;
+    p.tiles = std::max(1, (n + tile - 1) / tile);
     return p;
 }
 
+template <int Rounds>
 __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint32_t* __restrict__ keys, int n, int shift,
                                                         uint32_t mask, int tiles, int32_t* __restrict__ hist) {
     __shared__ int32_t cnt[kRsBins];
     for (int i = threadIdx.x; i < kRsBins; i += kRsThreads) cnt[i] = 0;
     __syncthreads();
-    const long base = (long)blockIdx.x * kRsTile;
-    for (int r = 0; r < kRsRounds; ++r) {
+    const long base = (long)blockIdx.x * (kRsThreads * Rounds);
+    for (int r = 0; r < Rounds; ++r) {
         const long i = base + (long)r * kRsThreads + threadIdx.x;
         if (i < n) atomicAdd(&cnt[(keys[i] >> shift) & mask], 1);
     }
@@ -121,6 +127,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scan(int32_t* __restrict__ hi
     if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
+template <int Rounds>
 __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t* __restrict__ keys_in,
                                                            const int32_t* __restrict__ vals_in, int n, int shift,
                                                            uint32_t mask, int tiles,
@@ -128,44 +135,72 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t* __res
                                                            const int32_t* __restrict__ totals,
                                                            uint32_t* __restrict__ keys_out,
                                                            int32_t* __restrict__ vals_out) {
-    __shared__ int32_t start[kRsBins];              // first output slot of each digit for this tile
-    __shared__ int32_t wcnt[kRsWarps][kRsBins];     // this round's count per warp and digit
+    __shared__ int32_t wcnt[kRsWarps][kRsBins];  // per warp: a digit's count, then the warps before it
+    __shared__ int32_t lstart[kRsBins];          // first place of each digit in the sorted tile
+    __shared__ int32_t gofs[kRsBins];            // output slot minus place in the tile
+    __shared__ uint32_t sk[kRsThreads * Rounds];
+    __shared__ int32_t sv[kRsThreads * Rounds];
     __shared__ int32_t warp_tot[kRsWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nd = (int)mask + 1;
-    {  // digit bases: exclusive scan of the totals (nd <= 256 = one per thread)
-        const int d = threadIdx.x;
-        int32_t total;
-        const int32_t ex = rs_block_scan(d < nd ? totals[d] : 0, total, warp_tot);
-        if (d < nd) start[d] = ex + hist[(long)d * tiles + blockIdx.x];
-    }
+    const long base = (long)blockIdx.x * (kRsThreads * Rounds);
+    const int cnt = (int)min((long)(kRsThreads * Rounds), (long)n - base);
     for (int i = threadIdx.x; i < kRsWarps * kRsBins; i += kRsThreads) (&wcnt[0][0])[i] = 0;
+    uint32_t k[Rounds];
+    int32_t v[Rounds], rank[Rounds];
+#pragma unroll
+    for (int r = 0; r < Rounds; ++r) {
+        const int i = (w * Rounds + r) * 32 + lane;
+        k[r] = i < cnt ? keys_in[base + i] : 0u;
+        v[r] = i < cnt ? vals_in[base + i] : 0;
+    }
     __syncthreads();
-    const long base = (long)blockIdx.x * kRsTile;
     const unsigned lt = (1u << lane) - 1u;
-    for (int r = 0; r < kRsRounds; ++r) {
-        const long i = base + (long)r * kRsThreads + threadIdx.x;
-        const bool live = i < n;
-        const uint32_t k = live ? keys_in[i] : 0u;
-        const int32_t v = live ? vals_in[i] : 0;
-        const int d = live ? (int)((k >> shift) & mask) : kRsBins;  // past the end: its own group
+#pragma unroll
+    for (int r = 0; r < Rounds; ++r) {
+        const bool live = (w * Rounds + r) * 32 + lane < cnt;
+        const int d = live ? (int)((k[r] >> shift) & mask) : kRsBins;  // past the end: its own group
         const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int rank_w = __popc(peers & lt);
-        const bool leader = rank_w == 0;
-        if (leader && live) wcnt[w][d] = __popc(peers);
-        __syncthreads();
-        if (live) {
-            int32_t pos = start[d] + rank_w;
-            for (int ww = 0; ww < w; ++ww) pos += wcnt[ww][d];
-            keys_out[pos] = k;
-            vals_out[pos] = v;
+        const int before = __popc(peers & lt);
+        rank[r] = live ? wcnt[w][d] + before : 0;
+        __syncwarp();
+        if (live && before == 0) wcnt[w][d] += __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    {  // one digit per thread (nd <= 256): its places in the tile and in the output
+        const int d = threadIdx.x;
+        int32_t in_tile = 0;
+        if (d < nd)
+#pragma unroll
+            for (int ww = 0; ww < kRsWarps; ++ww) {
+                const int32_t c = wcnt[ww][d];
+                wcnt[ww][d] = in_tile;
+                in_tile += c;
+            }
+        int32_t total;
+        const int32_t local = rs_block_scan(in_tile, total, warp_tot);
+        const int32_t first = rs_block_scan(d < nd ? totals[d] : 0, total, warp_tot);
+        if (d < nd) {
+            lstart[d] = local;
+            gofs[d] = first + hist[(long)d * tiles + blockIdx.x] - local;
         }
-        __syncthreads();
-        if (leader && live) {
-            atomicAdd(&start[d], wcnt[w][d]);
-            wcnt[w][d] = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < Rounds; ++r)
+        if ((w * Rounds + r) * 32 + lane < cnt) {
+            const int d = (int)((k[r] >> shift) & mask);
+            const int p = lstart[d] + wcnt[w][d] + rank[r];
+            sk[p] = k[r];
+            sv[p] = v[r];
         }
-        __syncthreads();
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt; i += kRsThreads) {
+        const uint32_t key = sk[i];
+        const int o = gofs[(key >> shift) & mask] + i;
+        keys_out[o] = key;
+        vals_out[o] = sv[i];
     }
 }
 
@@ -195,9 +230,10 @@ cudaError_t sort_pairs(void* temp, size_t temp_bytes, const uint32_t* keys_in, u
         uint32_t* ok = to_out ? keys_out : tk;
         int32_t* ov = to_out ? vals_out : tv;
         const int shift = pass * p.radix;
-        k_rs_hist<<<p.tiles, kRsThreads, 0, s>>>(ik, n, shift, mask, p.tiles, hist);
+        (p.rounds == 4 ? k_rs_hist<4> : k_rs_hist<16>)<<<p.tiles, kRsThreads, 0, s>>>(ik, n, shift, mask, p.tiles, hist);
         k_rs_scan<<<(int)mask + 1, kRsThreads, 0, s>>>(hist, p.tiles, totals);
-        k_rs_scatter<<<p.tiles, kRsThreads, 0, s>>>(ik, iv, n, shift, mask, p.tiles, hist, totals, ok, ov);
+        (p.rounds == 4 ? k_rs_scatter<4> : k_rs_scatter<16>)<<<p.tiles, kRsThreads, 0, s>>>(
+            ik, iv, n, shift, mask, p.tiles, hist, totals, ok, ov);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         ik = ok;
@@ -211,7 +247,8 @@ namespace {
 constexpr int kFlagThreads = 1024;  // slots per block of the flag and stayer kernels
 constexpr int kRankThreads = 256;
 constexpr int kSmallMovers = 32;    // movers placed by the last flag block (one warp each)
-constexpr int kMoverBlocks = 256;   // k_place_movers: 2,048 warps, a mover each (more: in turn)
+constexpr int kMoverBlocks = 1024;  // k_place_movers: 8,192 warps, a mover each, resident at once
+constexpr int kMoverTile = 1024;    // movers staged in shared memory at a time
 
 // first index i of the ascending a[0, n) with a[i] > k, found by one warp with
 // 32-way probes (about four dependent loads for a million entries)
@@ -265,6 +302,7 @@ __global__ void __launch_bounds__(kFlagThreads, 2) k_flag_movers(const uint32_t*
                                                               const uint32_t* __restrict__ prev, int n, int cap,
                                                               uint32_t* __restrict__ mask, int32_t* __restrict__ blk,
                                                               uint32_t* __restrict__ mk, int32_t* __restrict__ mj,
+                                                              uint32_t* __restrict__ mprev,
                                                               uint32_t* __restrict__ mkeys, int32_t* __restrict__ mslot,
                                                               int32_t* __restrict__ mpos,
                                                               int32_t* __restrict__ counters,
@@ -275,13 +313,14 @@ __global__ void __launch_bounds__(kFlagThreads, 2) k_flag_movers(const uint32_t*
     const int lane = threadIdx.x & 31;
     bool mover = false;
     if (j < n) {
-        const uint32_t k = keys[j];
-        mover = k != prev[j];
+        const uint32_t k = keys[j], pk = prev[j];
+        mover = k != pk;
         if (mover) {
             const int idx = atomicAdd(&counters[0], 1);
             if (idx < cap) {
                 mk[idx] = k;
                 mj[idx] = j;
+                mprev[idx] = pk;
             }
         }
     }
@@ -333,18 +372,53 @@ __global__ void __launch_bounds__(kFlagThreads, 2) k_flag_movers(const uint32_t*
     }
 }
 
-// placement of up to kBruteMovers movers, one warp each (grid-stride over the movers)
+// placement of up to kBruteMovers movers, one warp each (place_mover's ranks; the mover
+// list, its slots and their previous keys pass through shared memory once per block: read
+// from L2 by every warp, with prev[slot] behind the slot, the loads' latency made 8,192
+// movers cost more than a full sort).  Measured, 100,003 particles with a few thousand
+// movers: 20 -> 12 us per step with an ordering every 4th.
 __global__ void __launch_bounds__(kRankThreads) k_place_movers(const uint32_t* __restrict__ prev, int n, int cap,
                                                                const uint32_t* __restrict__ mk,
                                                                const int32_t* __restrict__ mj,
+                                                               const uint32_t* __restrict__ mprev,
                                                                const int32_t* __restrict__ counters,
                                                                uint32_t* __restrict__ mkeys, int32_t* __restrict__ mslot,
                                                                int32_t* __restrict__ mpos) {
-    const int m = counters[0];
+    __shared__ uint32_t sk[kMoverTile], sp[kMoverTile];
+    __shared__ int32_t sj[kMoverTile];
+    const int m = counters[0], lane = threadIdx.x & 31;
     if (m > cap || m > kBruteMovers) return;  // the full-sort branch (never launched with these)
-    const int warps = (int)(((long)gridDim.x * kRankThreads) >> 5);
-    for (int i = (int)(((long)blockIdx.x * kRankThreads + threadIdx.x) >> 5); i < m; i += warps)  // warp-uniform
-        place_mover(i, m, prev, n, mk, mj, mkeys, mslot, mpos, threadIdx.x & 31);
+    constexpr int kWarps = kRankThreads / 32;
+    for (int i0 = blockIdx.x * kWarps; i0 < m; i0 += gridDim.x * kWarps) {  // block-uniform
+        const int i = i0 + (threadIdx.x >> 5);
+        const bool live = i < m;
+        const uint32_t ki = live ? mk[i] : 0u;
+        const int ji = live ? mj[i] : 0;
+        int rank = 0, prev_le = 0;
+        for (int c0 = 0; c0 < m; c0 += kMoverTile) {
+            const int cn = min(kMoverTile, m - c0);
+            __syncthreads();
+            for (int k = threadIdx.x; k < cn; k += kRankThreads) {
+                sk[k] = mk[c0 + k];
+                sj[k] = mj[c0 + k];
+                sp[k] = mprev[c0 + k];
+            }
+            __syncthreads();
+            for (int k = lane; k < cn; k += 32) {
+                rank += (sk[k] < ki) | ((sk[k] == ki) & (sj[k] < ji));
+                prev_le += sp[k] <= ki;
+            }
+        }
+        rank = __reduce_add_sync(0xffffffffu, rank);
+        prev_le = __reduce_add_sync(0xffffffffu, prev_le);
+        if (!live) continue;
+        const int ub = warp_upper_bound(prev, n, ki, lane);
+        if (lane == 0) {
+            mkeys[rank] = ki;
+            mslot[rank] = ji;
+            mpos[rank] = rank + ub - prev_le;
+        }
+    }
 }
 
 // stayer j: (stayers before j) + (movers with key < key_j); threads t < m also
@@ -428,7 +502,7 @@ cudaError_t order_graph_build(void** out, cudaStream_t cs, const OrderBuffers& b
     OG_CK(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
     OG_CK(cudaStreamBeginCaptureToGraph(cs, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     OG_CK(cudaMemsetAsync(counters, 0, sizeof(int32_t), cs));
-    k_flag_movers<<<nb, kFlagThreads, 0, cs>>>(b.keys, b.keys_sorted, n, b.cap, mask, blk, b.mk, b.mj, b.mkeys,
+    k_flag_movers<<<nb, kFlagThreads, 0, cs>>>(b.keys, b.keys_sorted, n, b.cap, mask, blk, b.mk, b.mj, b.mprev, b.mkeys,
                                                b.mslot, b.mpos, counters, h, b.st);
     OG_CK(cudaGetLastError());
     cudaStreamCaptureStatus status;
@@ -447,7 +521,7 @@ cudaError_t order_graph_build(void** out, cudaStream_t cs, const OrderBuffers& b
     for (int c = 0; c < 2; ++c) {
         OG_CK(cudaStreamBeginCaptureToGraph(cs, body[c], nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
         if (c == 1)
-            k_place_movers<<<kMoverBlocks, kRankThreads, 0, cs>>>(b.keys_sorted, n, b.cap, b.mk, b.mj, counters,
+            k_place_movers<<<kMoverBlocks, kRankThreads, 0, cs>>>(b.keys_sorted, n, b.cap, b.mk, b.mj, b.mprev, counters,
                                                                   b.mkeys, b.mslot, b.mpos);
         k_place_stayers<<<nb, kFlagThreads, 0, cs>>>(b.keys, n, b.cap, mask, blk, b.mkeys, b.mslot, b.mpos, counters,
                                                      b.keys_sorted, b.perm);
