@@ -562,6 +562,7 @@ aep_status aep_solver_create(const aep_grid_desc* grid, const aep_params* params
     CK(cudaMalloc(&s->G.acc, sizeof(unsigned long long) * 4 * s->nnodes));
     CK(cudaMalloc(&s->G.vel, sizeof(float4) * s->nnodes));
     CK(cudaMalloc(&s->G.vbf, sizeof(float4) * s->nnodes));
+    CK(cudaMalloc(&s->G.vdiff, 2 * (size_t)s->nblocks));
     CK(cudaMalloc(&s->G.flag, sizeof(uint32_t) * (size_t)s->nblocks));
     CK(cudaMalloc(&s->G.active, sizeof(int32_t) * (size_t)s->nblocks));
     CK(cudaMalloc(&s->dstats, sizeof(DevStats)));
@@ -569,6 +570,7 @@ aep_status aep_solver_create(const aep_grid_desc* grid, const aep_params* params
     CK(cudaMemsetAsync(s->G.acc, 0, sizeof(unsigned long long) * 4 * s->nnodes, s->stream));
     CK(cudaMemsetAsync(s->G.vel, 0, sizeof(float4) * s->nnodes, s->stream));
     CK(cudaMemsetAsync(s->G.vbf, 0, sizeof(float4) * s->nnodes, s->stream));
+    CK(cudaMemsetAsync(s->G.vdiff, 0, 2 * (size_t)s->nblocks, s->stream));
     CK(cudaMemsetAsync(s->G.flag, 0, sizeof(uint32_t) * (size_t)s->nblocks, s->stream));
     CK(cudaMemsetAsync(s->dstats, 0, sizeof(DevStats), s->stream));
     CK(cudaStreamSynchronize(s->stream));
@@ -584,6 +586,7 @@ aep_status aep_solver_destroy(aep_solver* s) {
     cudaFree(s->G.acc);
     cudaFree(s->G.vel);
     cudaFree(s->G.vbf);
+    cudaFree(s->G.vdiff);
     cudaFree(s->G.flag);
     cudaFree(s->G.active);
     cudaFree(s->dstats);
@@ -1000,8 +1003,8 @@ aep_status step_impl(aep_solver* s, double dt_force, double dt, int32_t stage, b
         CKLAUNCH();
     }
     if (timed) mark(s, AEP_PHASE_CLOTH_G2P);
-    launch_cloth_g2p(s->kp, P, s->P[nx], s->G, M, (float)dt, s->keys, s->dstats, H, s->mlp ? &mp : nullptr,
-                     (float)s->learned_tol, (float)s->learned_abs, s->stream);
+    launch_cloth_g2p(s->kp, s->P[nx], M, s->keys, s->dstats, H, s->mlp ? &mp : nullptr, (float)s->learned_tol,
+                     (float)s->learned_abs, s->stream);
     CKLAUNCH();
     if (timed) {
         mark(s, AEP_NUM_PHASES);

@@ -100,6 +100,7 @@ struct GArrays {
     unsigned long long* acc;  // 4 per node: mass, momentum/impulse x, y, z (fixed point; acc_node)
     float4* vel;              // (v, m) after normalisation / after grid update
     float4* vbf;              // before-friction velocity (w unused)
+    uint8_t* vdiff;           // two per node block (32 nodes each): v and v^bf differ somewhere
     uint32_t* flag;           // per node block: touched this step
     int32_t* active;          // list of touched node blocks
     int32_t* nactive;         // its length
@@ -254,12 +255,7 @@ __device__ __forceinline__ void stencil_offsets(const KParams& P, const int base
     }
 }
 
-// Grid tile of a block of sorted particles: the 2x2x2 node blocks (512 nodes)
-// starting at the base-node block of the block's first particle.  Particles are
-// ordered by base-node block, so almost every particle of the block has its
-// whole 4x4x4 stencil inside; their gathers read shared memory instead of L1/L2.
-constexpr int kTileNodes = 512;
-
+// node block of a key
 __device__ __forceinline__ void tile_origin(const KParams& P, uint32_t key, int org[3]) {
     const uint32_t blk = key >> 6;
     org[0] = (int)(blk % (uint32_t)P.nb[0]);
@@ -282,40 +278,81 @@ __device__ __forceinline__ void pdl_entry() {
 }
 
 // asynchronous 4-byte copy global -> shared (cp.async; no registers held while in
-// flight), its commit and the wait for all of this thread's copies
+// flight) and the wait for all of this thread's copies
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// cooperative copy of the tile (all threads of the block); src2 / dst2 may be null
-__device__ __forceinline__ void load_tile(const KParams& P, const int org[3], const float4* __restrict__ src,
-                                          const float4* __restrict__ src2, float4* dst, float4* dst2) {
-    for (int i = threadIdx.x; i < kTileNodes; i += blockDim.x) {
-        const int t = i >> 6;
-        const uint32_t gblk = (uint32_t)(((org[2] + (t >> 2)) * P.nb[1] + org[1] + ((t >> 1) & 1)) * P.nb[0] + org[0] +
-                                         (t & 1));
-        const uint32_t node = (gblk << 6) | (uint32_t)(i & 63);
-        dst[i] = src[node];
-        if (dst2) dst2[i] = src2[node];
-    }
-}
+// The gathers' grid tile: the 13 x 9 x 9 nodes from one node before the node block of the
+// thread block's first particle, in plain x-fastest order.  The particles are ordered by
+// node block, x fastest: a block's 128 particles mostly sit in two x-adjacent node blocks,
+// and those that moved a cell since the last ordering in the cells around them, so one
+// lane in 50 and 3% of the warps leave the tile (a CPU count over ordered keys; 18% and
+// 43% with 2 x 2 x 2 node blocks).  In this order a node's offset from its stencil's base
+// is a constant, so the 64 loads of a gather need one address register.
+constexpr int kGtX = 13, kGtY = 9, kGtZ = 9, kGtNodes = kGtX * kGtY * kGtZ;
 
-// stencil offsets inside the tile when the stencil's base block is the tile's
-// origin (returns false otherwise); the same additive form as stencil_offsets
-__device__ __forceinline__ bool tile_offsets(const int base[3], const int org[3], uint32_t X[4], uint32_t Y[4],
-                                             uint32_t Z[4]) {
-    if ((base[0] >> 2) != org[0] || (base[1] >> 2) != org[1] || (base[2] >> 2) != org[2]) return false;
-#pragma unroll
-    for (int o = 0; o < 4; ++o) {
-        const int x = base[0] + o - 4 * org[0], y = base[1] + o - 4 * org[1], z = base[2] + o - 4 * org[2];
-        X[o] = (uint32_t)((x >> 2) * 64 + (x & 3));
-        Y[o] = (uint32_t)((y >> 2) * 128 + ((y & 3) << 2));
-        Z[o] = (uint32_t)((z >> 2) * 256 + ((z & 3) << 4));
-    }
-    return true;
+// asynchronous 16-byte copy global -> shared
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+// one node of the tile into shared memory (nothing outside the padded grid)
+__device__ __forceinline__ void load_gather_node(const KParams& P, const int org[3], const float4* __restrict__ src,
+                                                 float4* dst, int x, int y, int z) {
+    const int gx = 4 * org[0] - 1 + x, gy = 4 * org[1] - 1 + y, gz = 4 * org[2] - 1 + z;
+    if (gx >= 0 && gy >= 0 && gz >= 0 && gx < 4 * P.nb[0] && gy < 4 * P.nb[1] && gz < 4 * P.nb[2])
+        cp_async16(dst + (z * kGtY + y) * kGtX + x, src + node_index(P, gx, gy, gz));
+}
+// cooperative asynchronous copy of the tile by 128 threads (the caller waits for its
+// copies and synchronises): rows y < 8 of every z by 16 threads each, then the rows y = 8
+__device__ __forceinline__ void load_gather_tile(const KParams& P, const int org[3], const float4* __restrict__ src,
+                                                 float4* dst) {
+    const int x = threadIdx.x & 15, y = threadIdx.x >> 4;
+    if (x < kGtX)
+#pragma unroll 3
+        for (int z = 0; z < kGtZ; ++z) load_gather_node(P, org, src, dst, x, y, z);
+    if (threadIdx.x < kGtX * kGtZ) load_gather_node(P, org, src, dst, threadIdx.x % kGtX, 8, threadIdx.x / kGtX);
+}
+// whether the stencil from padded node `base` lies in the tile; its offset there
+__device__ __forceinline__ bool gather_offset(const int base[3], const int org[3], int& off) {
+    const int x = base[0] - 4 * org[0] + 1, y = base[1] - 4 * org[1] + 1, z = base[2] - 4 * org[2] + 1;
+    off = (z * kGtY + y) * kGtX + x;
+    return (unsigned)x <= kGtX - 4 && (unsigned)y <= kGtY - 4 && (unsigned)z <= kGtZ - 4;
+}
+// flag t (t < 72) of the node blocks under the tile, two per block: 4 x 3 x 3 blocks from
+// one before org
+__device__ __forceinline__ bool tile_differs(const KParams& P, const int org[3], const uint8_t* __restrict__ flags, int t) {
+    const int b = t >> 1, x = org[0] - 1 + (b & 3), y = org[1] - 1 + (b >> 2) % 3, z = org[2] - 1 + (b >> 2) / 3;
+    if (x < 0 || y < 0 || z < 0 || x >= P.nb[0] || y >= P.nb[1] || z >= P.nb[2]) return false;
+    return flags[2 * ((z * P.nb[1] + y) * P.nb[0] + x) + (t & 1)] != 0;
+}
+// whether one of the flags (tile_differs, all 72) covers a node of the stencil from `base`
+// inside the tile
+__device__ __forceinline__ bool stencil_differs(const int base[3], const int org[3], const uint8_t* flags) {
+    bool d = false;
+    const int x0 = (base[0] >> 2) - org[0] + 1, x1 = ((base[0] + 3) >> 2) - org[0] + 1;
+    const int y0 = (base[1] >> 2) - org[1] + 1, y1 = ((base[1] + 3) >> 2) - org[1] + 1;
+    const int z0 = (base[2] >> 1) - 2 * org[2] + 2, z1 = ((base[2] + 3) >> 1) - 2 * org[2] + 2;
+    for (int z = z0; z <= z1; ++z)
+        for (int y = y0; y <= y1; ++y)
+            for (int x = x0; x <= x1; ++x) d |= flags[2 * (((z >> 1) * 3 + y) * 4 + x) + (z & 1)] != 0;
+    return d;
+}
+// the same for any stencil, from the flags in global memory
+__device__ __forceinline__ bool grid_differs(const KParams& P, const int base[3], const uint8_t* __restrict__ flags) {
+    bool d = false;
+    for (int z = base[2] >> 1; z <= (base[2] + 3) >> 1; ++z)
+        for (int y = base[1] >> 2; y <= (base[1] + 3) >> 2; ++y)
+            for (int x = base[0] >> 2; x <= (base[0] + 3) >> 2; ++x)
+                d |= flags[2 * (((z >> 1) * P.nb[1] + y) * P.nb[0] + x) + (z & 1)] != 0;
+    return d;
+}
+// v[o], o = 0..3, without an indexed register array
+__device__ __forceinline__ float pick4(const float v[4], int o) {
+    return o < 2 ? (o == 0 ? v[0] : v[1]) : (o == 2 ? v[2] : v[3]);
 }
 
 // weights of one particle with the reference's out-of-grid node drop (HS:44-46)
@@ -607,12 +644,18 @@ __device__ __forceinline__ double dp_exp(double x) { return exp(x); }
 __device__ __forceinline__ float dp_sin(float x) { return __sinf(x); }
 __device__ __forceinline__ double dp_sin(double x) { return sin(x); }
 
+// sqrt(2/3) 2 sin(phi) / (3 - sin(phi)) at the hardened friction angle phi(q)
 template <typename T>
-__device__ __forceinline__ int dp_project(T ln[3], T& q, T h0, T h1, T h2, T h3, T k) {
+__device__ __forceinline__ T dp_alpha(T q, T h0, T h1, T h2, T h3) {
     const T deg = T(3.14159265358979323846 / 180.0);
     T phi = (h0 + (h1 * q - h3) * dp_exp(-h2 * q)) * deg;
     T sphi = dp_sin(phi);
-    T alpha = T(0.81649658092772603273) * T(2) * sphi / (T(3) - sphi);  // sqrt(2/3)
+    return T(0.81649658092772603273) * T(2) * sphi / (T(3) - sphi);  // sqrt(2/3)
+}
+
+template <typename T>
+__device__ __forceinline__ int dp_project(T ln[3], T& q, T h0, T h1, T h2, T h3, T k) {
+    T alpha = dp_alpha(q, h0, h1, h2, h3);
     T tr = ln[0] + ln[1] + ln[2];
     T dev[3] = {ln[0] - tr / T(3), ln[1] - tr / T(3), ln[2] - tr / T(3)};
     T nd = sqrt_t(dev[0] * dev[0] + dev[1] * dev[1] + dev[2] * dev[2]);

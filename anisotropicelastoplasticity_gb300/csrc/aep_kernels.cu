@@ -415,53 +415,88 @@ constexpr int kFrcRec = 11;
 constexpr int kFrcWarpBuf = 32 * kFrcRec + 1;
 __device__ __forceinline__ int frc_slot(int p) { return p * kFrcRec + (p >= 16 ? 1 : 0); }
 
+// Velocity gradient of the P2G velocity (the three SpMVs of HS:269-271), contracted one
+// axis at a time: Gm = sum v (grad w)^T with grad w = (dwx wy wz, wx dwy wz, wx wy dwz)
+__device__ __forceinline__ void gradient_row(const float4 v[4], const float wx[4], const float dx[4], float cz, float dz,
+                                             float B[3][3]) {
+    float Ad[3] = {0, 0, 0}, Aw[3] = {0, 0, 0};
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+        Ad[0] = fmaf(dx[o], v[o].x, Ad[0]); Ad[1] = fmaf(dx[o], v[o].y, Ad[1]); Ad[2] = fmaf(dx[o], v[o].z, Ad[2]);
+        Aw[0] = fmaf(wx[o], v[o].x, Aw[0]); Aw[1] = fmaf(wx[o], v[o].y, Aw[1]); Aw[2] = fmaf(wx[o], v[o].z, Aw[2]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        B[0][c] = fmaf(cz, Ad[c], B[0][c]);
+        B[1][c] = fmaf(cz, Aw[c], B[1][c]);
+        B[2][c] = fmaf(dz, Aw[c], B[2][c]);
+    }
+}
+__device__ __forceinline__ void gradient_add(const float B[3][3], float cy, float dy, float Gm[9]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        Gm[3 * c + 0] = fmaf(cy, B[0][c], Gm[3 * c + 0]);
+        Gm[3 * c + 1] = fmaf(dy, B[1][c], Gm[3 * c + 1]);
+        Gm[3 * c + 2] = fmaf(cy, B[2][c], Gm[3 * c + 2]);
+    }
+}
+// from the block's tile (t: the stencil's base node there); a loop over y as in gather_tile
+__device__ __forceinline__ void gradient_tile(const float4* t, const float w[3][4], const float dw[3][4], float Gm[9]) {
+    float wy[4], dy[4];
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+        wy[o] = w[1][o];
+        dy[o] = dw[1][o];
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Gm[k] = 0.f;
+#pragma unroll 1
+    for (int oy = 0; oy < 4; ++oy) {
+        float B[3][3] = {};
+#pragma unroll
+        for (int oz = 0; oz < 4; ++oz) {
+            const float4 v[4] = {t[oz * kGtX * kGtY], t[oz * kGtX * kGtY + 1], t[oz * kGtX * kGtY + 2],
+                                 t[oz * kGtX * kGtY + 3]};
+            gradient_row(v, w[0], dw[0], w[2][oz], dw[2][oz], B);
+        }
+        gradient_add(B, wy[0], dy[0], Gm);
+        t += kGtX;
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            wy[o] = wy[o + 1];
+            dy[o] = dy[o + 1];
+        }
+    }
+}
+// the same sums in the same order from the grid (stencils outside the tile)
+__device__ __forceinline__ void gradient_grid(const KParams& P, const float4* __restrict__ f, const int base[3],
+                                              const float w[3][4], const float dw[3][4], float Gm[9]) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Gm[k] = 0.f;
+#pragma unroll 1
+    for (int oy = 0; oy < 4; ++oy) {
+        float B[3][3] = {};
+#pragma unroll 1
+        for (int oz = 0; oz < 4; ++oz) {
+            float4 v[4];
+#pragma unroll
+            for (int o = 0; o < 4; ++o) v[o] = f[node_index(P, base[0] + o, base[1] + oy, base[2] + oz)];
+            gradient_row(v, w[0], dw[0], pick4(w[2], oz), pick4(dw[2], oz), B);
+        }
+        gradient_add(B, pick4(w[1], oy), pick4(dw[1], oy), Gm);
+    }
+}
+
 // The FP32 stress impulse of one particle; a near-degenerate F-hat (a singular
 // value under 2% of the largest) gives S = 0 here and the particle is listed for
 // k_force_fp64, which redoes it in FP64 and scatters it on its own (keeping the
 // FP64 code, and its registers, out of k_force).
-// vel: the grid velocities (global) or the block's tile; X, Y, Z the stencil
-// offsets into it; w, dw the particle's weights
+// Gm: the velocity gradient of the P2G velocity (gradient_tile).
 // F_E, the plastic scalar and the volume of the particle come from the caller's
 // shared-memory copies (sF[k][t], sq[t], svol[t]: copied while the grid tile loads)
-__device__ void particle_stress_impulse(const KParams& P, const float4* vel, const uint32_t X[4], const uint32_t Y[4],
-                                        const uint32_t Z[4], const PArrays& cur, int pj, int mat, const float* sF,
-                                        int t, int tstride, float q_in, float vol, float dt_force, float S[9],
-                                        const float w[3][4], const float dw[3][4], DevStats* st, int32_t* fp64_list,
-                                        int fp64_cap) {
-    // velocity gradient of the P2G velocity (the three SpMVs of HS:269-271),
-    // contracted one axis at a time: Gm = sum v (grad w)^T with
-    // grad w = (dwx wy wz, wx dwy wz, wx wy dwz)
-    float Gm[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int oy = 0; oy < 4; ++oy) {
-        float Bd[3] = {0, 0, 0}, Bw[3] = {0, 0, 0}, Bz[3] = {0, 0, 0};
-#pragma unroll
-        for (int oz = 0; oz < 4; ++oz) {
-            const uint32_t yz = Y[oy] + Z[oz];
-            float Ad[3] = {0, 0, 0}, Aw[3] = {0, 0, 0};
-#pragma unroll
-            for (int ox = 0; ox < 4; ++ox) {
-                const float4 v = vel[yz + X[ox]];
-                const float a = w[0][ox], d = dw[0][ox];
-                Ad[0] = fmaf(d, v.x, Ad[0]); Ad[1] = fmaf(d, v.y, Ad[1]); Ad[2] = fmaf(d, v.z, Ad[2]);
-                Aw[0] = fmaf(a, v.x, Aw[0]); Aw[1] = fmaf(a, v.y, Aw[1]); Aw[2] = fmaf(a, v.z, Aw[2]);
-            }
-            const float cz = w[2][oz], dz = dw[2][oz];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                Bd[c] = fmaf(cz, Ad[c], Bd[c]);
-                Bw[c] = fmaf(cz, Aw[c], Bw[c]);
-                Bz[c] = fmaf(dz, Aw[c], Bz[c]);
-            }
-        }
-        const float cy = w[1][oy], dy = dw[1][oy];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            Gm[3 * c + 0] = fmaf(cy, Bd[c], Gm[3 * c + 0]);
-            Gm[3 * c + 1] = fmaf(dy, Bw[c], Gm[3 * c + 1]);
-            Gm[3 * c + 2] = fmaf(cy, Bz[c], Gm[3 * c + 2]);
-        }
-    }
+__device__ void particle_stress_impulse(const KParams& P, const float Gm[9], const PArrays& cur, int pj, int mat,
+                                        const float* sF, int t, int tstride, float q_in, float vol, float dt_force,
+                                        float S[9], DevStats* st, int32_t* fp64_list, int fp64_cap) {
     float F[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) F[k] = sF[k * tstride + t];
@@ -567,16 +602,17 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
                                                        float dt_force, DevStats* st, MeshArrays M,
                                                        int32_t* fp64_list, int fp64_cap) {
     pdl_entry();
-    __shared__ float4 sm4[(kFrcThreads / 32) * kFrcWarpBuf];
-    __shared__ float4 tile_v[kTileNodes];
+    // the grid tile, then (after a barrier) the warps' prep records in the same memory
+    __shared__ float4 sm4[std::max((kFrcThreads / 32) * kFrcWarpBuf, kGtNodes)];
+    float4* const tile = sm4;
     dt_force = step_dt(P, dt_force, 0);
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float4* const buf = sm4 + wid * kFrcWarpBuf;
-    const long chunk0 = ((long)blockIdx.x * (kFrcThreads / 32) + wid) * 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float4* const buf = sm4 + warp * kFrcWarpBuf;
+    const long chunk0 = ((long)blockIdx.x * (kFrcThreads / 32) + warp) * 32;
     const long j = chunk0 + lane;
     int org[3];
     tile_origin(P, keys[(long)blockIdx.x * kFrcThreads], org);
-    load_tile(P, org, G.vel, nullptr, tile_v, nullptr);
+    load_gather_tile(P, org, G.vel, tile);
     // the particle's own loads and weights overlap the tile copy
     const bool live = j < n;
     const int pj = live ? perm[j] : 0;
@@ -589,31 +625,34 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
         for (int k = 0; k < 9; ++k) cp_async4(&sF[k][threadIdx.x], &cur.F[k][pj]);
         cp_async4(&sq[threadIdx.x], &cur.plastic[pj]);
         cp_async4(&svol[threadIdx.x], &cur.vol[pj]);
-        cp_async_commit();
     }
     int cell[3];
     float w[3][4], dw[3][4];
-    uint32_t X[4], Y[4], Z[4];
+    int toff = 0;
     bool in_tile = false;
     {
         float f[3];
         locate(P, cur.x[0][pj], cur.x[1][pj], cur.x[2][pj], cell, f);
         particle_weights(P, cell, f, w, dw);
         const int base[3] = {cell[0] + 3, cell[1] + 3, cell[2] + 3};
-        in_tile = tile_offsets(base, org, X, Y, Z);
-        if (!in_tile) stencil_offsets(P, base, X, Y, Z);
+        in_tile = gather_offset(base, org, toff);
     }
+    cp_async_wait_all();
     __syncthreads();
-    if (chunk0 >= n) return;
     uint32_t my_key = kInvalidKey;
+    float S[9];
+    float av[3] = {0.f, 0.f, 0.f};  // w-weighted impulse (cloth vertices)
     if (live) {
-        float S[9];
-        float av[3] = {0.f, 0.f, 0.f};  // w-weighted impulse (cloth vertices)
         if (mat <= kSand) {
-            cp_async_wait_all();
-            particle_stress_impulse(P, in_tile ? tile_v : G.vel, X, Y, Z, cur, pj, mat, &sF[0][0], threadIdx.x,
-                                    kFrcThreads, sq[threadIdx.x], svol[threadIdx.x], dt_force, S, w, dw, st, fp64_list,
-                                    fp64_cap);
+            float Gm[9];
+            if (in_tile) {
+                gradient_tile(tile + toff, w, dw, Gm);
+            } else {
+                const int base[3] = {cell[0] + 3, cell[1] + 3, cell[2] + 3};
+                gradient_grid(P, G.vel, base, w, dw, Gm);
+            }
+            particle_stress_impulse(P, Gm, cur, pj, mat, &sF[0][0], threadIdx.x, kFrcThreads, sq[threadIdx.x],
+                                    svol[threadIdx.x], dt_force, S, st, fp64_list, fp64_cap);
         } else {
             const int id = cur.id[pj];
             if (mat == kClothVertex) {
@@ -633,6 +672,10 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
                 for (int k = 0; k < 9; ++k) S[k] = es[k];
             }
         }
+    }
+    __syncthreads();  // every gather from the tile is done
+    if (chunk0 >= n) return;
+    if (live) {
         float4* r = buf + frc_slot(lane);
         r[0] = make_float4(S[0], S[1], S[2], S[3]);
         r[1] = make_float4(S[4], S[5], S[6], S[7]);
@@ -655,7 +698,7 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
     // at the end of the run (warp-uniform) the halves are added and half h adds
     // z-layers 2h, 2h + 1 to the grid
     const int h = lane >> 4, l = lane & 15, ox = l & 3, oy = l >> 2;
-    const int cnt = (int)max(0l, min(32l, (long)n - chunk0));
+    const int cnt = (int)min(32l, (long)n - chunk0);
     float fx[4] = {0, 0, 0, 0}, fy[4] = {0, 0, 0, 0}, fz[4] = {0, 0, 0, 0};
     // run heads: a particle whose key differs from the previous one's (any order)
     const uint32_t key_before = __shfl_up_sync(0xffffffffu, my_key, 1);
@@ -818,6 +861,9 @@ __global__ void k_grid(KParams P, GArrays G, float dt_force, int write_force, do
             }
             continue;  // force stage: leave velocities and accumulators untouched
         }
+        // the 32 nodes of this warp are one half of a node block
+        const bool diff = __any_sync(0xffffffffu, v4.x != bf.x || v4.y != bf.y || v4.z != bf.z);
+        if ((threadIdx.x & 31) == 0) G.vdiff[2 * blk + ((i >> 5) & 1)] = diff;
         G.vel[node] = v4;
         G.vbf[node] = bf;
         a[kAccX] = a[kAccY] = a[kAccZ] = 0;  // the mass is zero since the normalisation
@@ -968,9 +1014,7 @@ __device__ __forceinline__ void return_map(const KParams& P, int mat, T s[3], T&
 // the stretch is too large for this form), the projection (0 elastic, 1 sand apex,
 // 2 snow clamp / sand cone), and F_E from the projected ln s.
 template <typename T>
-__device__ __forceinline__ bool stretch_trial(const float F[9], const float D[9], T ln[3], T V[9]) {
-    T e[6];
-    trial_stretch(F, D, e);
+__device__ __forceinline__ bool stretch_trial(const T e[6], T ln[3], T V[9]) {
     const T n2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + T(2) * (e[3] * e[3] + e[4] * e[4] + e[5] * e[5]);
     if (!(n2 < T(0.25))) return false;
     T lam[3];
@@ -999,23 +1043,24 @@ __device__ __forceinline__ int stretch_project(const KParams& P, int mat, const 
     return dp_project<T>(lnn, q, T(P.sand_h0), T(P.sand_h1), T(P.sand_h2), T(P.sand_h3), T(P.sand_k));
 }
 
-// F_E, the plastic scalar and sig from the trial and projected log singular values
+// F_E, the plastic scalar and (want_sig, for F_P) sig from the trial and projected log
+// singular values
 template <typename T>
 __device__ __forceinline__ void stretch_finish(int mat, const float F[9], const float D[9], const T V[9],
                                                const T ln[3], const T lnn[3], bool plastic, T q_new, float& q,
-                                               float Fe[9], float sig[3]) {
+                                               float Fe[9], bool want_sig, float sig[3]) {
+    sig[0] = sig[1] = sig[2] = 0.0f;
     if (!plastic) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) Fe[k] = F[k] + D[k];
-        sig[0] = sig[1] = sig[2] = 0.0f;
         return;
     }
     T rho[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        rho[a] = expm1_t(lnn[a] - ln[a]);
-        sig[a] = (float)expm1_t(ln[a] - lnn[a]);
-    }
+    for (int a = 0; a < 3; ++a) rho[a] = expm1_t(lnn[a] - ln[a]);
+    if (want_sig)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) sig[a] = (float)expm1_t(ln[a] - lnn[a]);
     // M = V diag(rho) V^T, then F_E = F + (D + (F + D) M)
     T M[9];
 #pragma unroll
@@ -1040,13 +1085,13 @@ __device__ __forceinline__ void stretch_finish(int mat, const float F[9], const 
 
 // The whole mapping; returns the projection's kind, or -1 when the stretch is too
 // large for this form (the caller takes the SVD form); ln_tr / ln_new return the
-// log singular values, Vo the right singular vectors.
+// log singular values, Vo the right singular vectors; e the trial stretch C - I.
 template <typename T>
-__device__ __forceinline__ int stretch_return_map(const KParams& P, int mat, const float F[9], const float D[9],
-                                                  float& q, float Fe[9], float Vo[9], float sig[3], float ln_tr[3],
-                                                  float ln_new[3]) {
+__device__ __forceinline__ int stretch_return_map(const KParams& P, int mat, const T e[6], const float F[9],
+                                                  const float D[9], float& q, float Fe[9], float Vo[9], float sig[3],
+                                                  float ln_tr[3], float ln_new[3]) {
     T ln[3], lnn[3], V[9];
-    if (!stretch_trial<T>(F, D, ln, V)) return -1;
+    if (!stretch_trial<T>(e, ln, V)) return -1;
     T qq = q;
     const int kind = stretch_project<T>(P, mat, ln, lnn, qq);
 #pragma unroll
@@ -1056,7 +1101,7 @@ __device__ __forceinline__ int stretch_return_map(const KParams& P, int mat, con
     }
 #pragma unroll
     for (int k = 0; k < 9; ++k) Vo[k] = (float)V[k];
-    stretch_finish<T>(mat, F, D, V, ln, lnn, kind != 0, qq, q, Fe, sig);
+    stretch_finish<T>(mat, F, D, V, ln, lnn, kind != 0, qq, q, Fe, P.track_fp, sig);
     return kind;
 }
 
@@ -1086,69 +1131,115 @@ __device__ __forceinline__ int trial_kind(const KParams& P, int mat, const float
 // A sand trial state within reach of the apex of the Drucker-Prager cone: projected
 // onto the apex, or |tr ln s| within 1e-3 of |ln s| of the switch between apex and
 // cone (HybridSolver.cpp:652-663).  With the FP64 option these mappings run again in FP64.
-__device__ __forceinline__ bool near_apex(int kind, const float ln[3]) {
-    if (kind == 1) return true;
-    const float tr = ln[0] + ln[1] + ln[2];
-    return fabsf(tr) <= 1e-3f * sqrtf(ln[0] * ln[0] + ln[1] * ln[1] + ln[2] * ln[2]);
+__device__ __forceinline__ bool near_apex(int kind, float tr, float ln2) {
+    return kind == 1 || fabsf(tr) <= 1e-3f * sqrtf(ln2);
 }
 
-// Gather of v (G2P velocity + APIC) and v^bf (advection + velocity gradient) over
-// the 4x4x4 stencil, contracted one axis at a time because the weights are tensor
-// products: x first (A), then z (B), then y.
-//   A0 = sum_x wx v      A1 = sum_x wx xi_x v   A2 = sum_x dwx vbf   A3 = sum_x wx vbf
-//   vp = sum w v,  C = sum w v xi^T,  xs = sum w vbf,  Gb = sum vbf (grad w)^T
-__device__ __forceinline__ void g2p_gather(const float4* vel, const float4* vbf, const float w[3][4],
-                                           const float dw[3][4], const float xi[3][4], const uint32_t X[4],
-                                           const uint32_t Y[4], const uint32_t Z[4], float vp[3], float C[9],
-                                           float xs[3], float Gb[9]) {
+// Gather of a velocity field over the 4x4x4 stencil, contracted one axis at a time
+// because the weights are tensor products: x first (A), then z (B), then y.
+//   A0 = sum_x wx v      A1 = sum_x wx xi_x v   A2 = sum_x dwx v
+//   vp = sum w v,  C = sum w v xi^T,  Gb = sum v (grad w)^T
+// G2P takes vp and C from the velocity, xs = vp and Gb from the before-friction velocity;
+// where the two fields are equal (no node took the collision branch) one gather gives all.
+struct Gathered {
+    float vp[3], C[9], Gb[9];
+};
+// one z row of four nodes, added to the row sums B (weights wx, wxi, dwx; cz, czx, dz)
+__device__ __forceinline__ void gather_row(const float4 v[4], const float wx[4], const float wxi[4], const float dx[4],
+                                           float cz, float czx, float dz, float B[5][3]) {
+    float A0[3] = {0, 0, 0}, A1[3] = {0, 0, 0}, A2[3] = {0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < 3; ++k) vp[k] = xs[k] = 0.f;
+    for (int o = 0; o < 4; ++o) {
+        A0[0] = fmaf(wx[o], v[o].x, A0[0]); A0[1] = fmaf(wx[o], v[o].y, A0[1]); A0[2] = fmaf(wx[o], v[o].z, A0[2]);
+        A1[0] = fmaf(wxi[o], v[o].x, A1[0]); A1[1] = fmaf(wxi[o], v[o].y, A1[1]); A1[2] = fmaf(wxi[o], v[o].z, A1[2]);
+        A2[0] = fmaf(dx[o], v[o].x, A2[0]); A2[1] = fmaf(dx[o], v[o].y, A2[1]); A2[2] = fmaf(dx[o], v[o].z, A2[2]);
+    }
 #pragma unroll
-    for (int k = 0; k < 9; ++k) C[k] = Gb[k] = 0.f;
+    for (int c = 0; c < 3; ++c) {
+        B[0][c] = fmaf(cz, A0[c], B[0][c]);
+        B[1][c] = fmaf(cz, A1[c], B[1][c]);
+        B[2][c] = fmaf(czx, A0[c], B[2][c]);
+        B[3][c] = fmaf(cz, A2[c], B[3][c]);
+        B[4][c] = fmaf(dz, A0[c], B[4][c]);
+    }
+}
+__device__ __forceinline__ void gather_add(const float B[5][3], float cy, float cyx, float dy, Gathered& g) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        g.vp[c] = fmaf(cy, B[0][c], g.vp[c]);
+        g.C[3 * c + 0] = fmaf(cy, B[1][c], g.C[3 * c + 0]);
+        g.C[3 * c + 1] = fmaf(cyx, B[0][c], g.C[3 * c + 1]);
+        g.C[3 * c + 2] = fmaf(cy, B[2][c], g.C[3 * c + 2]);
+        g.Gb[3 * c + 0] = fmaf(cy, B[3][c], g.Gb[3 * c + 0]);
+        g.Gb[3 * c + 1] = fmaf(dy, B[0][c], g.Gb[3 * c + 1]);
+        g.Gb[3 * c + 2] = fmaf(cy, B[4][c], g.Gb[3 * c + 2]);
+    }
+}
+__device__ __forceinline__ void gather_zero(Gathered& g) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) g.vp[k] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) g.C[k] = g.Gb[k] = 0.f;
+}
+// From the block's tile (t: the stencil's base node there).  The y loop stays a loop (its
+// weights rotate through registers): unrolled over all 64 nodes, the ~1,500 instructions of
+// the gather (24 KB, each executed once per warp) made the instruction fetch a bound of
+// the pass (0.5 to 2.7 no-instruction stalls per issue).  Measured, with the tile, one gather
+// of both fields where no flag says that they differ, and cloth elements in the same pass:
+// G2P 92 -> 83 us for 524,288 sand particles at 128^3, 361 -> 299 for 2,097,152 of snow and
+// sand at 256^3, 1,448 -> 1,136 for 8,388,608 with cloth at 512^3.
+__device__ __forceinline__ void gather_tile(const float4* t, const float w[3][4], const float dw[3][4],
+                                            const float xi[3][4], Gathered& g) {
+    float wxi[4], wy[4], wyx[4], dy[4];
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+        wxi[o] = w[0][o] * xi[0][o];
+        wy[o] = w[1][o];
+        wyx[o] = w[1][o] * xi[1][o];
+        dy[o] = dw[1][o];
+    }
+    gather_zero(g);
+#pragma unroll 1
+    for (int oy = 0; oy < 4; ++oy) {
+        float B[5][3] = {};
+#pragma unroll
+        for (int oz = 0; oz < 4; ++oz) {
+            const float4 v[4] = {t[oz * kGtX * kGtY], t[oz * kGtX * kGtY + 1], t[oz * kGtX * kGtY + 2],
+                                 t[oz * kGtX * kGtY + 3]};
+            gather_row(v, w[0], wxi, dw[0], w[2][oz], w[2][oz] * xi[2][oz], dw[2][oz], B);
+        }
+        gather_add(B, wy[0], wyx[0], dy[0], g);
+        t += kGtX;
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            wy[o] = wy[o + 1];
+            wyx[o] = wyx[o + 1];
+            dy[o] = dy[o + 1];
+        }
+    }
+}
+// The same sums in the same order from the grid (stencils outside the tile, cloth
+// elements); rows one after another, small code for a rare path
+__device__ __forceinline__ void gather_grid(const KParams& P, const float4* __restrict__ f, const int base[3],
+                                            const float w[3][4], const float dw[3][4], const float xi[3][4],
+                                            Gathered& g) {
     float wxi[4];
 #pragma unroll
     for (int o = 0; o < 4; ++o) wxi[o] = w[0][o] * xi[0][o];
-#pragma unroll
+    gather_zero(g);
+#pragma unroll 1
     for (int oy = 0; oy < 4; ++oy) {
-        float B0[3] = {0, 0, 0}, B1[3] = {0, 0, 0}, B2[3] = {0, 0, 0};
-        float B3[3] = {0, 0, 0}, B4[3] = {0, 0, 0}, B5[3] = {0, 0, 0};
-#pragma unroll
+        float B[5][3] = {};
+#pragma unroll 1
         for (int oz = 0; oz < 4; ++oz) {
-            const uint32_t yz = Y[oy] + Z[oz];
-            float A0[3] = {0, 0, 0}, A1[3] = {0, 0, 0}, A2[3] = {0, 0, 0}, A3[3] = {0, 0, 0};
+            float4 v[4];
 #pragma unroll
-            for (int ox = 0; ox < 4; ++ox) {
-                const float4 v = vel[yz + X[ox]];
-                const float4 b = vbf[yz + X[ox]];
-                const float a = w[0][ox], ax_ = wxi[ox], d = dw[0][ox];
-                A0[0] = fmaf(a, v.x, A0[0]); A0[1] = fmaf(a, v.y, A0[1]); A0[2] = fmaf(a, v.z, A0[2]);
-                A1[0] = fmaf(ax_, v.x, A1[0]); A1[1] = fmaf(ax_, v.y, A1[1]); A1[2] = fmaf(ax_, v.z, A1[2]);
-                A2[0] = fmaf(d, b.x, A2[0]); A2[1] = fmaf(d, b.y, A2[1]); A2[2] = fmaf(d, b.z, A2[2]);
-                A3[0] = fmaf(a, b.x, A3[0]); A3[1] = fmaf(a, b.y, A3[1]); A3[2] = fmaf(a, b.z, A3[2]);
-            }
-            const float cz = w[2][oz], czx = w[2][oz] * xi[2][oz], dz = dw[2][oz];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                B0[c] = fmaf(cz, A0[c], B0[c]);
-                B1[c] = fmaf(cz, A1[c], B1[c]);
-                B2[c] = fmaf(czx, A0[c], B2[c]);
-                B3[c] = fmaf(cz, A2[c], B3[c]);
-                B4[c] = fmaf(cz, A3[c], B4[c]);
-                B5[c] = fmaf(dz, A3[c], B5[c]);
-            }
+            for (int o = 0; o < 4; ++o) v[o] = f[node_index(P, base[0] + o, base[1] + oy, base[2] + oz)];
+            const float cz = pick4(w[2], oz);
+            gather_row(v, w[0], wxi, dw[0], cz, cz * pick4(xi[2], oz), pick4(dw[2], oz), B);
         }
-        const float cy = w[1][oy], cyx = w[1][oy] * xi[1][oy], dy = dw[1][oy];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            vp[c] = fmaf(cy, B0[c], vp[c]);
-            C[3 * c + 0] = fmaf(cy, B1[c], C[3 * c + 0]);
-            C[3 * c + 1] = fmaf(cyx, B0[c], C[3 * c + 1]);
-            C[3 * c + 2] = fmaf(cy, B2[c], C[3 * c + 2]);
-            xs[c] = fmaf(cy, B4[c], xs[c]);
-            Gb[3 * c + 0] = fmaf(cy, B3[c], Gb[3 * c + 0]);
-            Gb[3 * c + 1] = fmaf(dy, B4[c], Gb[3 * c + 1]);
-            Gb[3 * c + 2] = fmaf(cy, B5[c], Gb[3 * c + 2]);
-        }
+        const float cy = pick4(w[1], oy);
+        gather_add(B, cy, cy * pick4(xi[1], oy), pick4(dw[1], oy), g);
     }
 }
 
@@ -1195,39 +1286,58 @@ __device__ __forceinline__ void harvest_record(const KParams& P, const Harvest& 
     for (int k = 0; k < 3; ++k) r[5 + k] = t[k] - srt[k];
 }
 
+constexpr int kG2PSmallPart = 64;  // particles per thread block of the small form
+
 // G2P + APIC + advection + F update + return mapping, one thread per particle.
 // kDefer (the learned return map): the trial state's yield check runs here; a
 // plastic snow or sand state whose projection is not a constant is queued (trial
 // ln s, D, V) for k_mlp_finish, which writes its F_E, F_P and plastic scalar;
 // elastic states and the sand apex are mapped exactly here.
-template <bool kDefer>
-__global__ void __launch_bounds__(128, 4) k_g2p(KParams P, PArrays cur, PArrays nxt, const int32_t* __restrict__ perm,
+// kSmall: 64 particles per block of 128 threads while the device holds all such blocks at
+// once (4 per SM).  There the kernel's time is the latency of one block; the particles of
+// a scattered block that miss its tile gather 64 nodes from L2, which is what takes longest
+// (4.8 of 14 us), so half the block's shared memory serves a second tile and each tile
+// half the particles.  Measured: 16.7 -> 13.4 us at 2,500 particles, 20.9 -> 18.7 at 16,000,
+// 18.2 -> 16.4 at 38,000; with twice the limit 22.0 -> 25.4 at 60,000.
+template <bool kDefer, bool kSmall>
+__global__ void __launch_bounds__(128, kSmall || !kDefer ? 4 : 5) k_g2p(KParams P, PArrays cur, PArrays nxt, const int32_t* __restrict__ perm,
                                              int n, GArrays G, float dt, uint32_t* __restrict__ keys_next,
                                              DevStats* st, Harvest H, const uint32_t* __restrict__ keys_sorted,
                                              MlpQueue Qu) {
     pdl_entry();
-    __shared__ float4 tile_v[kTileNodes], tile_b[kTileNodes];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    int org[3];
-    tile_origin(P, keys_sorted[blockIdx.x * blockDim.x], org);
-    load_tile(P, org, G.vel, G.vbf, tile_v, tile_b);
+    constexpr int kPart = kSmall ? kG2PSmallPart : 128;  // particles of the block
+    __shared__ float4 tile[kGtNodes], tile2[kSmall ? kGtNodes : 1];
+    __shared__ uint8_t sdiff[72];
+    const int j = blockIdx.x * kPart + threadIdx.x;
+    int org[3], org2[3] = {0, 0, 0};
+    bool has2 = false;
+    tile_origin(P, keys_sorted[blockIdx.x * kPart], org);
+    if (kSmall) tile_origin(P, keys_sorted[min((int)(blockIdx.x + 1) * kPart, n) - 1], org2);
+    load_gather_tile(P, org, G.vel, tile);
+    if (kSmall) {  // a second tile where the block's last particle is outside the first
+        has2 = org2[1] != org[1] || org2[2] != org[2] || (unsigned)(org2[0] - org[0]) > 1u;
+        if (has2) load_gather_tile(P, org2, G.vel, tile2);
+    }
+    // where v and v^bf differ under the tile (flags of the grid update): only the particles
+    // whose stencil reaches such a node gather v^bf too
+    const bool differ = threadIdx.x < 72 && tile_differs(P, org, G.vdiff, threadIdx.x);
+    if (threadIdx.x < 72) sdiff[threadIdx.x] = differ;
     // the particle's own loads and weights overlap the tile copy; F_E and the
     // per-particle scalars, read after the gather, are copied to shared memory
     // asynchronously meanwhile (each thread reads back only its own entries).  The
     // learned form (kDefer), with its queue code, loads them directly: it is at its
     // register limit already.
-    const bool live = j < n;
+    const bool live = j < n && threadIdx.x < kPart;
     const int pj = live ? perm[j] : 0;
-    __shared__ float sF[9][128], sq[128], sm[128], svol[128];
-    __shared__ int32_t sid[128];
-    if (!kDefer) {
+    __shared__ float sF[9][kPart], sq[kPart], sm[kPart], svol[kPart];
+    __shared__ int32_t sid[kPart];
+    if (!kDefer && threadIdx.x < kPart) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) cp_async4(&sF[k][threadIdx.x], &cur.F[k][pj]);
         cp_async4(&sq[threadIdx.x], &cur.plastic[pj]);
         cp_async4(&sm[threadIdx.x], &cur.m[pj]);
         cp_async4(&svol[threadIdx.x], &cur.vol[pj]);
         cp_async4(&sid[threadIdx.x], &cur.id[pj]);
-        cp_async_commit();
     }
     const int mat = live ? (int)cur.mat[pj] : (int)kClothElement;
     float xp[3] = {cur.x[0][pj], cur.x[1][pj], cur.x[2][pj]};
@@ -1236,24 +1346,65 @@ __global__ void __launch_bounds__(128, 4) k_g2p(KParams P, PArrays cur, PArrays 
     locate(P, xp[0], xp[1], xp[2], cell, f);
     const bool truncated = particle_weights(P, cell, f, w, dw);
     int base[3] = {cell[0] + 3, cell[1] + 3, cell[2] + 3};
-    uint32_t X[4], Y[4], Z[4];
-    const bool in_tile = tile_offsets(base, org, X, Y, Z);
-    if (!in_tile) stencil_offsets(P, base, X, Y, Z);
-    __syncthreads();
-    // elements follow their vertices (k_cloth_g2p)
-    if (!live || mat == kClothElement) {
-        cp_async_wait_all();  // no copy into this block's shared memory outlives the thread
-        return;
-    }
-    dt = step_dt(P, dt, 1);
+    int toff, toff2 = 0;
+    const bool in_tile = gather_offset(base, org, toff);
+    const bool in_tile2 = kSmall && !in_tile && has2 && gather_offset(base, org2, toff2);
+    const float4* const stencil = in_tile ? tile + toff : tile2 + toff2;
     float xi[3][4];
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int o = 0; o < 4; ++o) xi[a][o] = ((float)(o - 1) - f[a]) * P.h[a];
-
+    cp_async_wait_all();
+    const bool two = __syncthreads_or(differ);
+    const bool vbf2 = kSmall && two && !has2;  // the second buffer takes v^bf under the first tile
+    if (vbf2) load_gather_tile(P, org, G.vbf, tile2);  // arrives during the first gather
     float vp[3], xs[3], C[9], Gb[9];
-    g2p_gather(in_tile ? tile_v : G.vel, in_tile ? tile_b : G.vbf, w, dw, xi, X, Y, Z, vp, C, xs, Gb);
+    if (live) {
+        Gathered g;
+        if (in_tile || in_tile2) gather_tile(stencil, w, dw, xi, g);
+        else gather_grid(P, G.vel, base, w, dw, xi, g);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) vp[c] = xs[c] = g.vp[c];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            C[k] = g.C[k];
+            Gb[k] = g.Gb[k];
+        }
+    }
+    if (vbf2) {
+        cp_async_wait_all();
+        __syncthreads();
+    }
+    if (!live) return;
+    dt = step_dt(P, dt, 1);
+    if (in_tile ? two && stencil_differs(base, org, sdiff) : grid_differs(P, base, G.vdiff)) {
+        Gathered g;
+        if (vbf2 && in_tile) gather_tile(tile2 + toff, w, dw, xi, g);
+        else gather_grid(P, G.vbf, base, w, dw, xi, g);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) xs[c] = g.vp[c];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) Gb[k] = g.Gb[k];
+    }
+    if (mat == kClothElement) {
+        // APIC momenta (HS:927-933) and the trial d3 += dt grad v^bf d3 (HS:584-607), which
+        // k_cloth_g2p maps; position, velocity and d1, d2 follow the vertices there
+        float Bn[9];
+        apic_damp(C, P.mesh_damp, Bn);
+        const float d3o[3] = {cur.F[2][pj], cur.F[5][pj], cur.F[8][pj]};
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            nxt.F[3 * a + 2][j] = dt * (Gb[3 * a] * d3o[0] + Gb[3 * a + 1] * d3o[1] + Gb[3 * a + 2] * d3o[2]) + d3o[a];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) nxt.B[k][j] = Bn[k];
+        nxt.plastic[j] = cur.plastic[pj];
+        nxt.mat[j] = (uint8_t)mat;
+        nxt.m[j] = cur.m[pj];
+        nxt.vol[j] = cur.vol[pj];
+        nxt.id[j] = cur.id[pj];
+        return;
+    }
     // advection x = sum w (x_i + dt v^bf_i) (HS:944): exact linear reproduction for a
     // full stencil; a stencil cut by the grid boundary keeps its lost weight.
     float xn[3];
@@ -1295,11 +1446,9 @@ __global__ void __launch_bounds__(128, 4) k_g2p(KParams P, PArrays cur, PArrays 
         const bool vclamped = locate(P, xn[0], xn[1], xn[2], vc, vf);
         keys_next[j] = make_key(P, vc);
         if (vclamped) atomicAdd(&st->out_of_domain, 1ull);
-        cp_async_wait_all();
         return;
     }
     // F update (HS:560-576): F_tr = F + D, D = dt grad v^bf F
-    if (!kDefer) cp_async_wait_all();
     float F[9], GF[9], Ftr[9], D[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) F[k] = kDefer ? cur.F[k][pj] : sF[k][threadIdx.x];
@@ -1321,12 +1470,17 @@ __global__ void __launch_bounds__(128, 4) k_g2p(KParams P, PArrays cur, PArrays 
     int skind = -1;
     float sig[3];
     if (!kDefer) {
-        float lt[3], lnw[3];
+        float e[6];
+        trial_stretch(F, D, e);
         const float q_old = q;
-        skind = stretch_return_map<float>(P, mat, F, D, q, Fe, V, sig, lt, lnw);
-        if (skind >= 0 && P.fp64_apex && mat == kSand && near_apex(skind, lt)) {
+        float lt[3], lnw[3];
+        skind = stretch_return_map<float>(P, mat, e, F, D, q, Fe, V, sig, lt, lnw);
+        const float tr = lt[0] + lt[1] + lt[2], ln2 = lt[0] * lt[0] + lt[1] * lt[1] + lt[2] * lt[2];
+        if (skind >= 0 && P.fp64_apex && mat == kSand && near_apex(skind, tr, ln2)) {
             q = q_old;  // the same mapping again, in FP64
-            skind = stretch_return_map<double>(P, mat, F, D, q, Fe, V, sig, lt, lnw);
+            double ed[6];
+            trial_stretch(F, D, ed);
+            skind = stretch_return_map<double>(P, mat, ed, F, D, q, Fe, V, sig, lt, lnw);
             cg::coalesced_group g = cg::coalesced_threads();
             if (g.thread_rank() == 0) atomicAdd(&st->fp64_apex, (unsigned long long)g.size());
         }
@@ -1335,8 +1489,9 @@ __global__ void __launch_bounds__(128, 4) k_g2p(KParams P, PArrays cur, PArrays 
         // the learned return map: the trial state and its yield check here; a plastic
         // state with a projection the network predicts is queued for k_mlp_finish
         // (trial ln s, D, V), everything else is mapped exactly in place
-        float ln[3];
-        const bool in_range = stretch_trial<float>(F, D, ln, V);
+        float ln[3], e[6];
+        trial_stretch(F, D, e);
+        const bool in_range = stretch_trial<float>(e, ln, V);
         const int tk = in_range ? trial_kind(P, mat, ln, q) : -1;
         // the queue positions of the warp's plastic lanes: one atomic, issued here and
         // read after the exact mappings of its other lanes, which hide its round trip
@@ -1349,7 +1504,7 @@ __global__ void __launch_bounds__(128, 4) k_g2p(KParams P, PArrays cur, PArrays 
             if (tk != 2) {
                 float lnn[3], qq = q;
                 const int kind = stretch_project<float>(P, mat, ln, lnn, qq);
-                stretch_finish<float>(mat, F, D, V, ln, lnn, kind != 0, qq, q, Fe, sig);
+                stretch_finish<float>(mat, F, D, V, ln, lnn, kind != 0, qq, q, Fe, P.track_fp, sig);
                 if (kind == 1) {
                     cg::coalesced_group g = cg::coalesced_threads();  // the apex: exact, counted
                     if (g.thread_rank() == 0) atomicAdd(&st->learned_exact, (unsigned long long)g.size());
@@ -1598,7 +1753,7 @@ __global__ void __launch_bounds__(kFinThreads) k_mlp_finish(KParams P, PArrays c
                 D[k] = f[(kQD + k) * cap];
                 V[k] = f[(kQV + k) * cap];
             }
-            stretch_finish<float>(mat, F, D, V, ln, lnn, true, q_new, q, Fe, sig);
+            stretch_finish<float>(mat, F, D, V, ln, lnn, true, q_new, q, Fe, P.track_fp, sig);
             const int j = Qu.j[r];
 #pragma unroll
             for (int k = 0; k < 9; ++k) nxt.F[k][j] = Fe[k];
@@ -1632,56 +1787,38 @@ __global__ void __launch_bounds__(kFinThreads) k_mlp_finish(KParams P, PArrays c
 }
 
 // ===================================================================================
-// cloth elements (one thread per element): APIC momenta from the element's own
-// G2P velocity at its old centroid (HS:927-933), velocity = mean of the new vertex
-// velocities (HS:749-756), position = centroid of the new vertex positions
-// (LagrangianMesh.cpp:371-380), directions d1, d2 from the vertices and
-// d3 += dt grad v^bf d3 (HS:584-607), then the QR return mapping (HS:686-720).
-// With an MLP (use_mlp), the cloth return mapping of plastic elements (shear beyond
+// cloth elements (one thread per element): velocity = mean of the new vertex velocities
+// (HS:749-756), position = centroid of the new vertex positions (LagrangianMesh.cpp:371-380),
+// directions d1, d2 from the vertices, d3 the trial that k_g2p left (HS:584-607), then the
+// QR return mapping (HS:686-720).  The element's own grid gather runs in k_g2p, from its
+// tile and in the order of the grid blocks: here, a thread per element in mesh order read
+// 128 nodes from L2 (205 -> 60 us of this kernel for the cloth among 8,388,608 particles
+// at 512^3, 39 -> 13 for the 196,608-particle drape).
+// With an MLP (kMlp), the cloth return mapping of plastic elements (shear beyond
 // the frictional cap) is predicted by the learned map (cloth rows of the same
 // network) and checked against the cap's optimality conditions, the exact
 // projection replacing a rejected prediction; the warp runs the network when any
 // of its elements is plastic.  With a harvest buffer (plain steps), plastic
 // elements record [r13, r23, r33 - 1, cap ratio, 2, projected - trial (3)].
-__global__ void __launch_bounds__(128) k_cloth_g2p(KParams P, PArrays cur, PArrays nxt, GArrays G, MeshArrays M,
-                                                   float dt, uint32_t* __restrict__ keys_next, DevStats* st,
-                                                   Harvest H, MlpParams mlp, int use_mlp, float tol_rel,
-                                                   float tol_abs) {
+template <bool kMlp>
+__global__ void __launch_bounds__(128) k_cloth_g2p(KParams P, PArrays nxt, MeshArrays M,
+                                                   uint32_t* __restrict__ keys_next, DevStats* st, Harvest H,
+                                                   MlpParams mlp, float tol_rel, float tol_abs) {
     pdl_entry();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = e < M.nf;
-    dt = step_dt(P, dt, 1);
     MlpSmem W{};
-    if (use_mlp) {  // block-uniform
+    if (kMlp) {
         W = mlp_smem_carve(smem_raw);
         mlp_load_smem(mlp, W, threadIdx.x, blockDim.x);
         __syncthreads();
     }
     float Q[9], r[3] = {0, 0, 1}, rp[3] = {0, 0, 1}, cap = 0.0f;
     bool plastic = false, tension = false;
-    int j = 0, pc = 0;
+    int j = 0;
     if (live) {
-        const int id = M.ebase + e;
-        j = M.slot_of[id];
-        pc = M.curidx_of[id];
-        float xp[3] = {cur.x[0][pc], cur.x[1][pc], cur.x[2][pc]};
-        int cell[3];
-        float f[3], w[3][4], dw[3][4];
-        locate(P, xp[0], xp[1], xp[2], cell, f);
-        particle_weights(P, cell, f, w, dw);
-        int base[3] = {cell[0] + 3, cell[1] + 3, cell[2] + 3};
-        uint32_t X[4], Y[4], Z[4];
-        stencil_offsets(P, base, X, Y, Z);
-        float xi[3][4];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int o = 0; o < 4; ++o) xi[a][o] = ((float)(o - 1) - f[a]) * P.h[a];
-        float vp[3], xs[3], C[9], Gb[9];
-        g2p_gather(G.vel, G.vbf, w, dw, xi, X, Y, Z, vp, C, xs, Gb);
-        float Bn[9];
-        apic_damp(C, P.mesh_damp, Bn);
+        j = M.slot_of[M.ebase + e];
         float xv[3][3], vv[3][3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -1693,12 +1830,11 @@ __global__ void __launch_bounds__(128) k_cloth_g2p(KParams P, PArrays cur, PArra
             }
         }
         float D[9];
-        const float d3o[3] = {cur.F[2][pc], cur.F[5][pc], cur.F[8][pc]};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             D[3 * a + 0] = xv[1][a] - xv[0][a];
             D[3 * a + 1] = xv[2][a] - xv[0][a];
-            D[3 * a + 2] = dt * (Gb[3 * a] * d3o[0] + Gb[3 * a + 1] * d3o[1] + Gb[3 * a + 2] * d3o[2]) + d3o[a];
+            D[3 * a + 2] = nxt.F[3 * a + 2][j];
         }
         float R[9];
         gram_schmidt(D, Q, R);
@@ -1710,10 +1846,10 @@ __global__ void __launch_bounds__(128) k_cloth_g2p(KParams P, PArrays cur, PArra
         cap = cloth_cap_ratio(r, M.shear, M.stiffness, M.friction);
         plastic = !tension && cap < 1.0f;
         // the exact projection, unless the learned map predicts this row
-        if (!(use_mlp && plastic)) cloth_project(rp, M.shear, M.stiffness, M.friction);
+        if (!(kMlp && plastic)) cloth_project(rp, M.shear, M.stiffness, M.friction);
         // records of states within 1e-5 of r = e3 would carry the FP32 rounding of
         // r33 as more than 1e-2 of their size: skipped
-        if (H.buf && !use_mlp && plastic && (e % H.stride) == 0 &&
+        if (H.buf && !kMlp && plastic && (e % H.stride) == 0 &&
             fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fabsf(r[2] - 1.0f)) >= 1e-5f) {
             const unsigned long long slot = atomicAdd(H.count, 1ull);
             if ((long long)slot < H.capacity) {
@@ -1729,23 +1865,16 @@ __global__ void __launch_bounds__(128) k_cloth_g2p(KParams P, PArrays cur, PArra
             nxt.x[a][j] = xn[a];
             nxt.v[a][j] = (vv[0][a] + vv[1][a] + vv[2][a]) / 3.0f;
         }
-#pragma unroll
-        for (int k = 0; k < 9; ++k) nxt.B[k][j] = Bn[k];
         nxt.F[0][j] = D[0]; nxt.F[1][j] = D[1];
         nxt.F[3][j] = D[3]; nxt.F[4][j] = D[4];
         nxt.F[6][j] = D[6]; nxt.F[7][j] = D[7];
-        nxt.plastic[j] = cur.plastic[pc];
-        nxt.mat[j] = (uint8_t)kClothElement;
-        nxt.m[j] = cur.m[pc];
-        nxt.vol[j] = cur.vol[pc];
-        nxt.id[j] = id;
         int nc[3];
         float nf[3];
         const bool clamped = locate(P, xn[0], xn[1], xn[2], nc, nf);
         keys_next[j] = make_key(P, nc);
         if (clamped) atomicAdd(&st->out_of_domain, 1ull);
     }
-    if (use_mlp) {
+    if (kMlp) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         unsigned char* wbase = smem_raw + kMlpSmemBytes + warp * kMlpWarpBytes;
         __nv_bfloat16* MX = reinterpret_cast<__nv_bfloat16*>(wbase);
@@ -2189,12 +2318,18 @@ void launch_g2p(const KParams& P, const PArrays& cur, const PArrays& nxt, const 
                 const GArrays& G, float dt, uint32_t* keys_next, DevStats* st, cudaStream_t s, const Harvest& H,
                 bool learned, const uint32_t* keys_sorted, const MlpQueue& Qu) {
     if (n <= 0) return;
-    if (learned)
-        launch_pdl(k_g2p<true>, blocks_for(n, 128), 128, 0, s, P, cur, nxt, perm, n, G, dt, keys_next, st, H,
-                   keys_sorted, Qu);
-    else
-        launch_pdl(k_g2p<false>, blocks_for(n, 128), 128, 0, s, P, cur, nxt, perm, n, G, dt, keys_next, st, H,
-                   keys_sorted, Qu);
+    // the small form while its blocks fit the device at once
+    static const int slots = [] {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        return std::max(1, sms) * 4;
+    }();
+    const bool small = (n + kG2PSmallPart - 1) / kG2PSmallPart <= slots;
+    const auto kernel = learned ? (small ? k_g2p<true, true> : k_g2p<true, false>)
+                                : (small ? k_g2p<false, true> : k_g2p<false, false>);
+    launch_pdl(kernel, blocks_for(n, small ? kG2PSmallPart : 128), 128, 0, s, P, cur, nxt, perm, n, G, dt, keys_next,
+               st, H, keys_sorted, Qu);
 }
 void launch_mlp_finish(const KParams& P, const PArrays& cur, const PArrays& nxt, const MlpQueue& Qu, DevStats* st,
                        const MlpParams& mlp, float tol_rel, float tol_abs, cudaStream_t s) {
@@ -2212,21 +2347,22 @@ void launch_mlp_finish(const KParams& P, const PArrays& cur, const PArrays& nxt,
     const int blocks = std::min(blocks_for(Qu.cap, kFinThreads), resident);
     launch_pdl(k_mlp_finish, blocks, kFinThreads, smem, s, P, cur, nxt, Qu, st, mlp, tol_rel, tol_abs);
 }
-void launch_cloth_g2p(const KParams& P, const PArrays& cur, const PArrays& nxt, const GArrays& G, const MeshArrays& M,
-                      float dt, uint32_t* keys_next, DevStats* st, const Harvest& H, const MlpParams* mlp,
-                      float tol_rel, float tol_abs, cudaStream_t s) {
+void launch_cloth_g2p(const KParams& P, const PArrays& nxt, const MeshArrays& M, uint32_t* keys_next, DevStats* st,
+                      const Harvest& H, const MlpParams* mlp, float tol_rel, float tol_abs, cudaStream_t s) {
     if (M.nf <= 0) return;
     constexpr int kClothMlpSmem = kMlpSmemBytes + 4 * kMlpWarpBytes;
-    const int smem = mlp ? kClothMlpSmem : 0;
-    if (mlp) {
-        static const bool attr_set = [] {  // once per process, before the first learned launch
-            cudaFuncSetAttribute(k_cloth_g2p, cudaFuncAttributeMaxDynamicSharedMemorySize, kClothMlpSmem);
-            return true;
-        }();
-        (void)attr_set;
+    if (!mlp) {
+        launch_pdl(k_cloth_g2p<false>, blocks_for(M.nf, 128), 128, 0, s, P, nxt, M, keys_next, st, H, MlpParams{},
+                   tol_rel, tol_abs);
+        return;
     }
-    launch_pdl(k_cloth_g2p, blocks_for(M.nf, 128), 128, smem, s, P, cur, nxt, G, M, dt, keys_next, st, H,
-               mlp ? *mlp : MlpParams{}, mlp ? 1 : 0, tol_rel, tol_abs);
+    static const bool attr_set = [] {  // once per process, before the first learned launch
+        cudaFuncSetAttribute(k_cloth_g2p<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClothMlpSmem);
+        return true;
+    }();
+    (void)attr_set;
+    launch_pdl(k_cloth_g2p<true>, blocks_for(M.nf, 128), 128, kClothMlpSmem, s, P, nxt, M, keys_next, st, H, *mlp,
+               tol_rel, tol_abs);
 }
 void launch_volumes(const KParams& P, const PArrays& cur, const int32_t* perm, int n, const GArrays& G,
                     cudaStream_t s) {

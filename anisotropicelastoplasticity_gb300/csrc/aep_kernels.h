@@ -25,9 +25,8 @@ void launch_g2p(const KParams& P, const PArrays& cur, const PArrays& nxt, const 
                 bool learned, const uint32_t* keys_sorted, const MlpQueue& queue);
 void launch_mlp_finish(const KParams& P, const PArrays& cur, const PArrays& nxt, const MlpQueue& queue, DevStats* st,
                        const MlpParams& mlp, float tol_rel, float tol_abs, cudaStream_t s);
-void launch_cloth_g2p(const KParams& P, const PArrays& cur, const PArrays& nxt, const GArrays& G, const MeshArrays& M,
-                      float dt, uint32_t* keys_next, DevStats* st, const Harvest& H, const MlpParams* mlp,
-                      float tol_rel, float tol_abs, cudaStream_t s);
+void launch_cloth_g2p(const KParams& P, const PArrays& nxt, const MeshArrays& M, uint32_t* keys_next, DevStats* st,
+                      const Harvest& H, const MlpParams* mlp, float tol_rel, float tol_abs, cudaStream_t s);
 void launch_volumes(const KParams& P, const PArrays& cur, const int32_t* perm, int n, const GArrays& G,
                     cudaStream_t s);
 void launch_upload(int n, int mode, const double* src, float* const* dst, cudaStream_t s,
