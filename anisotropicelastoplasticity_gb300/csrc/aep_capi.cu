@@ -355,7 +355,6 @@ const void* device_source(aep_solver* s, const void* p, size_t bytes, size_t off
                           bool* on_device = nullptr) {
     const void* a = device_alias(p, on_device);
     if (a) return a;
-    if (on_device) *on_device = true;
     double* st = s->staging + off;
     *err = cudaMemcpyAsync(st, p, bytes, cudaMemcpyHostToDevice, s->stream);
     return st;
@@ -403,6 +402,11 @@ aep_status download(aep_solver* s, double* dst, int count, int mode, float* cons
     if (sync) CK(cudaStreamSynchronize(s->stream));
     return AEP_OK;
 }
+
+// Readback into device memory goes by way of records from this many values per item: a
+// record costs 27 x 4 + 2 x 128 bytes whatever is asked for, a value read on its own a
+// 32-byte sector.
+constexpr int kRecordValues = 12;
 
 aep_status check_overflow(aep_solver* s) {
     DevStats h;
@@ -657,7 +661,8 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
     // in one launch, read back with the final synchronisation
     CK(cudaMemsetAsync(s->check, 0, 2 * sizeof(unsigned long long), s->stream));
     if (keep_order && all_on_device) {
-        launch_upload_slots((int)s->n, (int)n, src, P, s->prm.track_plastic_F, s->check, s->stream);
+        // by way of records, in the staging buffer (16 of its 37 doubles per item; unused here)
+        launch_upload_records((int)s->n, (int)n, src, P, s->prm.track_plastic_F, s->staging, s->check, s->stream);
     } else {
         // host memory is read in its own order, whole lines over the link
         const int32_t* map = nullptr;
@@ -1393,33 +1398,34 @@ aep_status aep_get_particles(aep_solver* s, int64_t n, double* x, double* v, dou
     aep_status st;
     const int64_t np = s->np;
     const size_t N = (size_t)np;
-    if ((st = prepare_download(s))) return st;
-    // one conversion launch for the requested fields (matrices into device memory in their
-    // own): straight into page-locked or
-    // device destinations, through staging (doubles: x 0, v 3N, B 6N, Fe 15N,
-    // Fp 24N, vol 33N, plastic 34N) and one copy each for pageable ones
+    // one conversion launch for the requested fields: straight into page-locked or device
+    // destinations, through staging (doubles: x 0, v 3N, B 6N, Fe 15N, Fp 24N, vol 33N,
+    // plastic 34N) and one copy each for pageable ones
     double* const req[7] = {x, v, B, Fe, Fp, vol, plastic};
     const size_t cnt[7] = {3, 3, 9, 9, 9, 1, 1}, off[7] = {0, 3, 6, 15, 24, 33, 34};
     double* dev[7] = {};
+    bool all_on_device = true;
+    int values = 0;  // of the record, per item
     for (int f = 0; f < 7; ++f)
         if (req[f]) {
             bool on_device = false;
             double* a = static_cast<double*>(const_cast<void*>(device_alias(req[f], &on_device)));
             dev[f] = a ? a : s->staging + off[f] * N;
-            if ((f == 3 || f == 4) && (on_device || !a)) {  // matrices in device memory leave from the slots' order
-                launch_download_F_slots((int)s->n, (int)np, dev[f], f == 3 ? P.F : P.Fp, P.id, s->stream);
-                CKLAUNCH();
-                if (!a)
-                    CK(cudaMemcpyAsync(req[f], dev[f], sizeof(double) * cnt[f] * N, cudaMemcpyDeviceToHost, s->stream));
-                dev[f] = nullptr;
-            }
+            all_on_device &= on_device;
+            values += f == 4 ? 0 : (int)cnt[f];
         }
-    DownloadDst dst{dev[0], dev[1], dev[2], dev[3], dev[4], dev[5], dev[6]};
-    launch_download_particles((int)np, dst, P, s->inv, s->stream);
-    CKLAUNCH();
-    for (int f = 0; f < 7; ++f)
-        if (dev[f] && dev[f] == s->staging + off[f] * N)
-            CK(cudaMemcpyAsync(req[f], dev[f], sizeof(double) * cnt[f] * N, cudaMemcpyDeviceToHost, s->stream));
+    const DownloadDst dst{dev[0], dev[1], dev[2], dev[3], dev[4], dev[5], dev[6]};
+    if (all_on_device && values >= kRecordValues) {
+        launch_download_records((int)s->n, (int)np, dst, P, s->staging, s->stream);
+        CKLAUNCH();
+    } else {
+        if ((st = prepare_download(s))) return st;
+        launch_download_particles((int)np, dst, P, s->inv, s->stream);
+        CKLAUNCH();
+        for (int f = 0; f < 7; ++f)
+            if (dev[f] && dev[f] == s->staging + off[f] * N)
+                CK(cudaMemcpyAsync(req[f], dev[f], sizeof(double) * cnt[f] * N, cudaMemcpyDeviceToHost, s->stream));
+    }
     CK(cudaStreamSynchronize(s->stream));
     return AEP_OK;
 }

@@ -1973,22 +1973,24 @@ __global__ void k_volumes(KParams P, PArrays cur, const int32_t* __restrict__ pe
 
 // ===================================================================================
 // layout conversion: reference FP64 layouts <-> device FP32 structure of arrays.
-// One thread per item and group of fields (blockIdx.y: the group, the slow index, so one
-// group's arrays fill the L2 while it runs); no thread divides.  The device's item order is
-// random against the caller's, so one side of every copy is random:
-//   caller's order (k_upload_particles, k_download_particles, k_upload, k_download):
-//     consecutive threads take consecutive items of the caller, so page-locked host memory
+// The device's item order is random against the caller's, so one side of every copy is random:
+//   host memory (k_upload_particles, k_download_particles, k_upload, k_download): one thread
+//     per item and group of fields (blockIdx.y: the group, the slow index, so one group's
+//     arrays fill the L2 while it runs), in the caller's order, so page-locked host memory
 //     streams over the host link at full width; the 3x3 matrices, 72 bytes per item, pass
 //     through shared memory for the same reason.
-//   slot order (k_upload_slots, k_download_F_slots), for arrays in device memory: the
-//     device side is coalesced and the random side moves whole doubles (or 72-byte
-//     matrices).  A scatter of 4-byte values costs a partial 32-byte sector each, and the
-//     L2 takes only 27 to 50 of those per clock (measured); reads of random doubles hit
-//     sectors that are shared by four items while a field is in the L2.
-// Measured, 7,604,222 particles + 784,386 cloth items on device arrays: upload 3.7 -> 2.05 ms,
-// readback 2.8 -> 2.3 ms (with the caller's own FP64 -> FP32 pass).
+//   device memory (k_pack_items + k_items_to_slots, k_slots_to_items + k_unpack_items): by
+//     way of 128-byte FP32 records, one per item in the caller's order.  The caller's arrays
+//     and the device's are then both read and written in order, and the random side moves
+//     whole records, four full sectors each; single values would cost a 32-byte sector each
+//     (15 of the 27 values of an item are columns of N x 3 arrays), and the L2 takes only 27
+//     to 50 partial sectors per clock (measured).
+// Measured, 7,604,222 particles + 784,386 cloth items on device arrays: upload 3.7 ms for one kernel
+// in the caller's order, 2.05 for one in slot order, 1.08 for records; readback (with the
+// caller's own FP64 -> FP32 pass) 2.8, 2.4 and 1.7 ms; 2,097,152 particles: upload and readback
+// 0.96 ms in slot order, 0.73 for records; 262,144: 0.24 for both
 constexpr int kConvThreads = 256;
-// fields per group: as many as the L2 holds of the randomly read side
+// fields per group of the readback in the caller's order: as many as the L2 holds
 constexpr long kConvL2Bytes = 48l << 20;
 
 // host-layout doubles -> FP32, one field set; item q goes to slot map[q] (or q).
@@ -2016,21 +2018,19 @@ __global__ void __launch_bounds__(kConvThreads) k_upload(int n, int mode, const 
     for (int i = 0; i < 3; ++i) d.f[conv_field(mode, g, i)][p] = (float)src[conv_index(mode, n, g, i, q)];
 }
 
-// m, vol, plastic, material and snow J_P of one item: the checks' inputs are returned
-__device__ __forceinline__ void upload_item(const UploadSrc& src, const PArrays& P, int q, int p, int track_fp,
-                                            unsigned long long& mx, unsigned long long& bad) {
+// m, vol, plastic (snow: J_P) and material of one item, FP32; the checks' inputs are returned
+struct ItemFields {
+    float m, vol, plastic;
+    int mat;
+};
+__device__ __forceinline__ ItemFields item_fields(const UploadSrc& src, int q, int track_fp, unsigned long long& mx,
+                                                  unsigned long long& bad) {
     const double m = src.m[q];
     if (!(m >= 0.0) || !isfinite(m)) bad = 1ull;
     else if (m > 0.0) mx = (unsigned long long)__double_as_longlong(m);
     const int mat = src.mat ? (int)src.mat[q] : kSand;
     if (mat > kSand) bad = 1ull;
-    P.m[p] = (float)m;
-    P.vol[p] = src.vol ? (float)src.vol[q] : 0.0f;
-    P.mat[p] = (uint8_t)mat;
     float pl = src.plastic ? (float)src.plastic[q] : 0.0f;
-    if (track_fp && !src.Fp)
-#pragma unroll
-        for (int c = 0; c < 9; ++c) P.Fp[c][p] = (c % 4 == 0) ? 1.0f : 0.0f;
     if (!track_fp && mat == kSnow) {  // J_P = det F_P, else the given scalar, else 1
         if (src.Fp) {
             double A[9];
@@ -2041,7 +2041,16 @@ __device__ __forceinline__ void upload_item(const UploadSrc& src, const PArrays&
             pl = 1.0f;
         }
     }
-    P.plastic[p] = pl;
+    return {(float)m, src.vol ? (float)src.vol[q] : 0.0f, pl, mat};
+}
+__device__ __forceinline__ void store_item(const PArrays& P, int p, const ItemFields& it, bool unit_fp) {
+    P.m[p] = it.m;
+    P.vol[p] = it.vol;
+    P.mat[p] = (uint8_t)it.mat;
+    P.plastic[p] = it.plastic;
+    if (unit_fp)
+#pragma unroll
+        for (int c = 0; c < 9; ++c) P.Fp[c][p] = (c % 4 == 0) ? 1.0f : 0.0f;
 }
 // check = {max mass bits, bad mass or tag}; all lanes call it
 __device__ __forceinline__ void upload_check(unsigned long long mx, unsigned long long bad, unsigned long long* check) {
@@ -2071,7 +2080,7 @@ __global__ void __launch_bounds__(kConvThreads) k_upload_particles(int n, Upload
         unsigned long long mx = 0ull, bad = 0ull;
         if (live) {
             P.id[p] = q;
-            upload_item(src, P, q, p, track_fp, mx, bad);
+            store_item(P, p, item_fields(src, q, track_fp, mx, bad), track_fp && !src.Fp);
         }
         upload_check(mx, bad, check);
     } else if (g > 5) {
@@ -2092,32 +2101,171 @@ __global__ void __launch_bounds__(kConvThreads) k_upload_particles(int n, Upload
     }
 }
 
-// The same into the slots the particles occupy now (P.id), from device arrays: one thread
-// per slot of all `slots` items (those of a mesh, ids n and above, are skipped).  Groups:
-// ceil(15 / per) of the planar fields x, v, B, then the item fields, Fe, F_P.
-__global__ void __launch_bounds__(kConvThreads) k_upload_slots(int slots, int n, int per, UploadSrc src, PArrays P,
-                                                               int track_fp, unsigned long long* check) {
-    const int p = blockIdx.x * kConvThreads + threadIdx.x, g = blockIdx.y, planar = (15 + per - 1) / per;
-    const int q = p < slots ? P.id[p] : n;
-    const bool live = q < n;
-    const long N = n;
-    if (g == planar) {  // block-uniform
-        unsigned long long mx = 0ull, bad = 0ull;
-        if (live) upload_item(src, P, q, p, track_fp, mx, bad);
-        upload_check(mx, bad, check);
-    } else if (!live) {
-    } else if (g > planar) {
-        const double* f = (g == planar + 1 ? src.Fe : src.Fp) + 9l * q;
+// Records of 32 words per item: x 0, v 3, B 6 (rows), F_E 15 (row-major), m 24, vol 25,
+// plastic 26, material 27.  A warp's 32 records pass through shared memory, chunk c (16
+// bytes) of record t at t * 8 + (c ^ (t & 7)): whole records on one side, one record per
+// lane on the other, both without bank conflicts.
+constexpr int kRecThreads = 128;
+struct ItemRecord {
+    float w[32];
+};
+__device__ __forceinline__ void record_to_shared(float4* sm, int t, const ItemRecord& r) {
 #pragma unroll
-        for (int c = 0; c < 9; ++c) (g == planar + 1 ? P.F : P.Fp)[3 * (c % 3) + c / 3][p] = (float)f[c];
-    } else {
-        for (int k = g * per; k < min(15, (g + 1) * per); ++k) {
-            const double* f = k < 3 ? src.x : k < 6 ? src.v : src.B;
-            const int c = k < 3 ? k : k < 6 ? k - 3 : k - 6;
-            float* d = k < 3 ? P.x[c] : k < 6 ? P.v[c] : P.B[c];
-            d[p] = f ? (float)f[c * N + q] : 0.0f;
+    for (int c = 0; c < 8; ++c)
+        sm[t * 8 + (c ^ (t & 7))] = make_float4(r.w[4 * c], r.w[4 * c + 1], r.w[4 * c + 2], r.w[4 * c + 3]);
+}
+__device__ __forceinline__ void record_from_shared(const float4* sm, int t, ItemRecord& r) {
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+        const float4 v = sm[t * 8 + (c ^ (t & 7))];
+        r.w[4 * c] = v.x; r.w[4 * c + 1] = v.y; r.w[4 * c + 2] = v.z; r.w[4 * c + 3] = v.w;
+    }
+}
+// the warp's records between shared memory and rec; q: the lane's record (>= n: none)
+template <bool kStore>
+__device__ __forceinline__ void move_records(float4* sm, float4* __restrict__ rec, int q, int n) {
+    const int lane = threadIdx.x & 31, c = lane & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = 4 * i + (lane >> 3), qt = __shfl_sync(0xffffffffu, q, t);
+        if (qt < n) {
+            if (kStore) rec[8l * qt + c] = sm[t * 8 + (c ^ (t & 7))];
+            else sm[t * 8 + (c ^ (t & 7))] = rec[8l * qt + c];
         }
     }
+}
+
+// the caller's device arrays into records, with the checks of the upload
+__global__ void __launch_bounds__(kRecThreads) k_pack_items(int n, UploadSrc src, float4* __restrict__ rec,
+                                                            int track_fp, unsigned long long* check) {
+    __shared__ float4 sm4[8 * kRecThreads];
+    __shared__ float sf[9 * kRecThreads];
+    const int w0 = threadIdx.x & ~31, lane = threadIdx.x & 31;
+    const int q0 = blockIdx.x * kRecThreads + w0, q = q0 + lane;
+    const long N = n;
+    float* const f = sf + 9 * w0;
+    const int words = 9 * max(0, min(32, n - q0));
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        if (32 * k + lane < words) f[32 * k + lane] = (float)src.Fe[9l * q0 + 32 * k + lane];
+    __syncwarp();
+    unsigned long long mx = 0ull, bad = 0ull;
+    if (q < n) {
+        ItemRecord r;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            r.w[c] = (float)src.x[c * N + q];
+            r.w[3 + c] = src.v ? (float)src.v[c * N + q] : 0.0f;
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            r.w[6 + c] = src.B ? (float)src.B[c * N + q] : 0.0f;
+            r.w[15 + 3 * (c % 3) + c / 3] = f[9 * lane + c];
+        }
+        const ItemFields it = item_fields(src, q, track_fp, mx, bad);
+        r.w[24] = it.m; r.w[25] = it.vol; r.w[26] = it.plastic; r.w[27] = __int_as_float(it.mat);
+#pragma unroll
+        for (int c = 28; c < 32; ++c) r.w[c] = 0.0f;
+        record_to_shared(sm4 + 8 * w0, lane, r);
+    }
+    upload_check(mx, bad, check);
+    __syncwarp();
+    move_records<true>(sm4 + 8 * w0, rec, q, n);
+}
+
+// records into the slots the particles occupy now (P.id), one thread per slot of all `slots`
+// items (those of a mesh, ids n and above, are skipped)
+__global__ void __launch_bounds__(kRecThreads) k_items_to_slots(int slots, int n, float4* __restrict__ rec, PArrays P,
+                                                                int unit_fp) {
+    __shared__ float4 sm4[8 * kRecThreads];
+    const int p = blockIdx.x * kRecThreads + threadIdx.x, w0 = threadIdx.x & ~31, lane = threadIdx.x & 31;
+    const int q = p < slots ? P.id[p] : n;
+    move_records<false>(sm4 + 8 * w0, rec, q, n);
+    __syncwarp();
+    if (q >= n) return;
+    ItemRecord r;
+    record_from_shared(sm4 + 8 * w0, lane, r);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        P.x[c][p] = r.w[c];
+        P.v[c][p] = r.w[3 + c];
+    }
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        P.B[c][p] = r.w[6 + c];
+        P.F[c][p] = r.w[15 + c];
+    }
+    store_item(P, p, {r.w[24], r.w[25], r.w[26], __float_as_int(r.w[27])}, unit_fp);
+}
+
+// F_P from a device array into the slots: 72 bytes per item
+__global__ void __launch_bounds__(kConvThreads) k_upload_F_slots(int slots, int n, const double* __restrict__ src,
+                                                                 FieldPtrs F, const int32_t* __restrict__ id) {
+    const int p = blockIdx.x * kConvThreads + threadIdx.x;
+    const int q = p < slots ? id[p] : n;
+    if (q >= n) return;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) F.f[3 * (c % 3) + c / 3][p] = (float)src[9l * q + c];
+}
+
+// the slots' state into records
+__global__ void __launch_bounds__(kRecThreads) k_slots_to_items(int slots, int n, PArrays P, float4* __restrict__ rec) {
+    __shared__ float4 sm4[8 * kRecThreads];
+    const int p = blockIdx.x * kRecThreads + threadIdx.x, w0 = threadIdx.x & ~31, lane = threadIdx.x & 31;
+    const int q = p < slots ? P.id[p] : n;
+    if (q < n) {
+        ItemRecord r;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            r.w[c] = P.x[c][p];
+            r.w[3 + c] = P.v[c][p];
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            r.w[6 + c] = P.B[c][p];
+            r.w[15 + c] = P.F[c][p];
+        }
+        r.w[24] = 0.0f; r.w[25] = P.vol[p]; r.w[26] = P.plastic[p];
+#pragma unroll
+        for (int c = 27; c < 32; ++c) r.w[c] = 0.0f;
+        record_to_shared(sm4 + 8 * w0, lane, r);
+    }
+    __syncwarp();
+    move_records<true>(sm4 + 8 * w0, rec, q, n);
+}
+
+// records into the caller's device arrays (the requested ones)
+__global__ void __launch_bounds__(kRecThreads) k_unpack_items(int n, float4* __restrict__ rec, DownloadDst dst) {
+    __shared__ float4 sm4[8 * kRecThreads];
+    __shared__ float sf[9 * kRecThreads];
+    const int w0 = threadIdx.x & ~31, lane = threadIdx.x & 31;
+    const int q0 = blockIdx.x * kRecThreads + w0, q = q0 + lane;
+    const long N = n;
+    float* const f = sf + 9 * w0;
+    move_records<false>(sm4 + 8 * w0, rec, q, n);
+    __syncwarp();
+    if (q < n) {
+        ItemRecord r;
+        record_from_shared(sm4 + 8 * w0, lane, r);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (dst.x) dst.x[c * N + q] = (double)r.w[c];
+            if (dst.v) dst.v[c * N + q] = (double)r.w[3 + c];
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            if (dst.B) dst.B[c * N + q] = (double)r.w[6 + c];
+            f[9 * lane + c] = r.w[15 + 3 * (c % 3) + c / 3];
+        }
+        if (dst.vol) dst.vol[q] = (double)r.w[25];
+        if (dst.plastic) dst.plastic[q] = (double)r.w[26];
+    }
+    __syncwarp();
+    if (!dst.Fe) return;
+    const int words = 9 * max(0, min(32, n - q0));
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        if (32 * k + lane < words) dst.Fe[9l * q0 + 32 * k + lane] = (double)f[32 * k + lane];
 }
 
 // The particle readback of aep_get_particles, in the caller's order: one thread per item
@@ -2422,13 +2570,22 @@ void launch_upload_particles(int n, const UploadSrc& src, const PArrays& P, cons
         k_upload_particles<<<conv_grid(n, (track_fp && src.Fp) ? 8 : 7), kConvThreads, 0, s>>>(n, src, P, map,
                                                                                                track_fp, check);
 }
-void launch_upload_slots(int slots, int n, const UploadSrc& src, const PArrays& P, int track_fp,
-                         unsigned long long* check, cudaStream_t s) {
-    // three 8-byte fields at a time while they fit the L2, else one (at 7.6 M particles
-    // three are 183 MB)
-    const int per = 24l * n <= kConvL2Bytes ? 3 : 1;
-    const int groups = (15 + per - 1) / per + ((track_fp && src.Fp) ? 3 : 2);
-    if (slots > 0) k_upload_slots<<<conv_grid(slots, groups), kConvThreads, 0, s>>>(slots, n, per, src, P, track_fp, check);
+void launch_upload_records(int slots, int n, const UploadSrc& src, const PArrays& P, int track_fp, void* rec,
+                           unsigned long long* check, cudaStream_t s) {
+    if (n <= 0) return;
+    float4* const r = static_cast<float4*>(rec);
+    k_pack_items<<<blocks_for(n, kRecThreads), kRecThreads, 0, s>>>(n, src, r, track_fp, check);
+    k_items_to_slots<<<blocks_for(slots, kRecThreads), kRecThreads, 0, s>>>(slots, n, r, P, track_fp && !src.Fp);
+    if (track_fp && src.Fp)
+        k_upload_F_slots<<<blocks_for(slots, kConvThreads), kConvThreads, 0, s>>>(slots, n, src.Fp, field_ptrs(P.Fp, 2),
+                                                                                  P.id);
+}
+void launch_download_records(int slots, int n, const DownloadDst& dst, const PArrays& P, void* rec, cudaStream_t s) {
+    if (n <= 0) return;
+    float4* const r = static_cast<float4*>(rec);
+    k_slots_to_items<<<blocks_for(slots, kRecThreads), kRecThreads, 0, s>>>(slots, n, P, r);
+    k_unpack_items<<<blocks_for(n, kRecThreads), kRecThreads, 0, s>>>(n, r, dst);
+    if (dst.Fp) launch_download_F_slots(slots, n, dst.Fp, P.Fp, P.id, s);
 }
 void launch_download_particles(int n, const DownloadDst& dst, const PArrays& P, const int32_t* inv, cudaStream_t s) {
     unsigned groups = 0;
@@ -2442,7 +2599,7 @@ void launch_download_particles(int n, const DownloadDst& dst, const PArrays& P, 
     add(dst.vol || dst.plastic, 5, 1);
     add(dst.Fe, 6, 1);
     add(dst.Fp, 7, 1);
-    const int split = 12l * n <= kConvL2Bytes ? 0 : 1;  // three 4-byte fields, as in launch_upload_slots
+    const int split = 12l * n <= kConvL2Bytes ? 0 : 1;  // three 4-byte fields
     if (n > 0 && count > 0)
         k_download_particles<<<conv_grid(n, split ? 3 * count : count), kConvThreads, 0, s>>>(n, groups, split, dst, P,
                                                                                               inv);

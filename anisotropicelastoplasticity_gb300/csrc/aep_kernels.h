@@ -42,8 +42,9 @@ struct DownloadDst {
 };
 void launch_upload_particles(int n, const UploadSrc& src, const PArrays& P, const int32_t* map, int track_fp,
                              unsigned long long* check, cudaStream_t s);
-void launch_upload_slots(int slots, int n, const UploadSrc& src, const PArrays& P, int track_fp,
-                         unsigned long long* check, cudaStream_t s);
+void launch_upload_records(int slots, int n, const UploadSrc& src, const PArrays& P, int track_fp, void* rec,
+                           unsigned long long* check, cudaStream_t s);
+void launch_download_records(int slots, int n, const DownloadDst& dst, const PArrays& P, void* rec, cudaStream_t s);
 void launch_download_F_slots(int slots, int n, double* dst, float* const* F, const int32_t* id, cudaStream_t s);
 void launch_download_particles(int n, const DownloadDst& dst, const PArrays& P, const int32_t* inv, cudaStream_t s);
 void launch_fixed_vertices(const KParams& P, const PArrays& cur, const GArrays& G, const MeshArrays& M,

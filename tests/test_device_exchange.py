@@ -1,4 +1,4 @@
-"""State exchange with arrays in device memory (slot order) against host arrays (the
+"""State exchange with arrays in device memory against host arrays (the
 caller's order): both convert the same FP64 values, so they agree bit for bit."""
 from __future__ import annotations
 
@@ -80,6 +80,28 @@ def test_device_arrays_match_host_arrays(n, fp, mesh):
     for a, b in zip(host, _get(s, n, fp, np.empty)):
         if a is not None:
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [31, 129, 4097])
+@pytest.mark.parametrize("want", ["x", "xv", "B", "xF", "vB", "Fq", "FP", "xvBFPVq"])
+def test_device_readback_of_some_fields(n, want):
+    """Any subset of the fields, by way of records (12 values per item and more) or each on
+    its own, gives the values that the host readback gives."""
+    import torch
+
+    sc = scenes.snow_block(n=8, res=32)
+    sc.params.track_plastic_F = 1
+    s = HybridSolver(None, sc.grid, sc.params)
+    s.set_level_set(sc.levelset)
+    _set(s, n, _state(n, True, 3))
+    s.step(1e-5)
+    host = _get(s, n, True, np.empty)
+    out = [torch.full((k * n,), 7.0, dtype=torch.float64, device="cuda") for k in (3, 3, 9, 9, 9, 1, 1)]
+    asked = [o if c in want else None for o, c in zip(out, "xvBFPVq")]
+    torch.cuda.synchronize()
+    assert s._lib.aep_get_particles(s._h, n, *[_ptr(a) for a in asked]) == capi.AEP_OK
+    for a, b, c in zip(host, out, "xvBFPVq"):
+        np.testing.assert_array_equal(b.cpu().numpy(), a if c in want else np.full(len(a), 7.0))
 
 
 def test_device_arrays_bad_mass_is_refused():
