@@ -4,8 +4,8 @@
 //                      cores (mma.sync bf16, f32 accumulation); each block writes its
 //                      weight and bias gradients to its own row of a partial array
 //   k_mlp_reduce     : sums the partial rows in block order (training is
-//                      deterministic: the same records give the same parameters)
-//   k_mlp_adam       : Adam on the f32 master parameters, refreshes the bf16 copies
+//                      deterministic: the same records give the same parameters); Adam
+//                      on the f32 master parameters, refreshes the bf16 copies
 //   k_mlp_infer      : batched forward pass (32 rows per warp), as used inside G2P
 // Training records (harvested from the exact return mapping where it changed the
 // state, 8 floats each):
@@ -46,40 +46,48 @@ constexpr int kTrainWarps = kTrainThreads / 32;
 
 using bf16 = __nv_bfloat16;
 
-__device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi) {
-    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+// as ldmatrix_x4, each 8x8 matrix transposed: register j of lane l holds rows 2(l%4),
+// 2(l%4)+1 of column l/4
+__device__ __forceinline__ void ldmatrix_x4_t(const bf16* p, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"(a));
 }
 
-// generic 16x8 tile: c += sum_{k < K} A(m0+i, k) B(k, n0+j); element (i,k) of A at
-// A[i*ars + k*acs] for i < am (zero otherwise), element (k,j) of B at B[k*brs + j*bcs]
-// for k < kmax (zero otherwise).  Used by training, where operands are transposed.
-template <int K>
-__device__ __forceinline__ void tile_mma(float c[4], const bf16* A, int ars, int acs, int am, const bf16* B, int brs,
-                                         int bcs, int kmax, int m0, int n0, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-    const bf16 z = __float2bfloat16(0.0f);
-    auto la = [&](int i, int k) { return (i < am && k < kmax) ? A[i * ars + k * acs] : z; };
-    auto lb = [&](int k, int j) { return k < kmax ? B[k * brs + j * bcs] : z; };
+// A 16x32 strip of four 16x8 tiles: c[j] += sum_{k < K} A(m0+i, k) B(k, n0+8j+i'), the k
+// tiles in order.  kAT false: A row-major at A[i * as + k], true: A[k * as + i];
+// kBT false: B column-major at B[j * bs + k], true: B[k * bs + j].
+template <bool kAT, bool kBT, int K>
+__device__ __forceinline__ void strip_mma(float (&c)[4][4], const bf16* A, int as, int m0, const bf16* B, int bs,
+                                          int n0, int lane) {
+    const int i = lane & 7, lo = (lane >> 3) & 1, hi = lane >> 4;
 #pragma unroll
     for (int k0 = 0; k0 < K; k0 += 16) {
-        const int r0 = m0 + g, r1 = m0 + g + 8, ka = k0 + 2 * t;
-        uint32_t a0 = pack2(la(r0, ka), la(r0, ka + 1)), a1 = pack2(la(r1, ka), la(r1, ka + 1));
-        uint32_t a2 = pack2(la(r0, ka + 8), la(r0, ka + 9)), a3 = pack2(la(r1, ka + 8), la(r1, ka + 9));
-        uint32_t b0 = pack2(lb(ka, n0 + g), lb(ka + 1, n0 + g)), b1 = pack2(lb(ka + 8, n0 + g), lb(ka + 9, n0 + g));
-        mma_bf16(c, a0, a1, a2, a3, b0, b1);
+        uint32_t a[4], b[8];
+        if (kAT) ldmatrix_x4_t(A + (k0 + i + 8 * hi) * as + m0 + 8 * lo, a[0], a[1], a[2], a[3]);
+        else ldmatrix_x4(A + (m0 + i + 8 * lo) * as + k0 + 8 * hi, a[0], a[1], a[2], a[3]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (kBT) ldmatrix_x4_t(B + (k0 + i + 8 * lo) * bs + n0 + 16 * h + 8 * hi, b[4 * h], b[4 * h + 1], b[4 * h + 2], b[4 * h + 3]);
+            else ldmatrix_x4(B + (n0 + 16 * h + i + 8 * hi) * bs + k0 + 8 * lo, b[4 * h], b[4 * h + 1], b[4 * h + 2], b[4 * h + 3]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_bf16(c[j], a[0], a[1], a[2], a[3], b[2 * j], b[2 * j + 1]);
     }
 }
 
-// 114,480 bytes: two blocks fit on an SM
-struct TrainSmem {
-    bf16 W1[64 * 16], W2[64 * 64], W3[64 * 64], W4[8 * 64];  // W^T, dense rows (the layout of the bf16 copy)
-    float b[200];
-    bf16 X[kTrainRows * 16];
-    bf16 H[3][kTrainRows * 64];   // post-activations
-    float Z[3][kTrainRows * 64];  // pre-activations
-    float T[kTrainRows * 4];
+// 87,136 bytes: two blocks fit on an SM.  Rows of 24 and 72 halves: the eight rows of an
+// ldmatrix lie on distinct banks.
+struct __align__(16) TrainSmem {
+    bf16 W1[64 * kStrideIn], W2[64 * kStrideH], W3[64 * kStrideH], W4[8 * kStrideH];  // W^T
+    bf16 X[kTrainRows * kStrideIn];
+    bf16 H[3][kTrainRows * kStrideH];   // post-activations
+    bf16 dZ[3][kTrainRows * kStrideH];  // of the layers 1..3
     bf16 dY[kTrainRows * 8];
-    bf16 dZ[2][kTrainRows * 64];  // ping-pong
+    float b[200];
+    float T[kTrainRows * 4];
+    float g1[64 * 17];  // W1's gradient, before its hi and lo columns are added
     float wloss[kTrainWarps];
 };
 
@@ -91,76 +99,97 @@ __device__ __forceinline__ float dsilu(float z) {
 // Forward and backward of one block of rows.  The block's gradient (f32, packed)
 // goes to its own row of `part` and its loss to part_loss[block]; k_mlp_reduce
 // sums the rows in block order, so training repeats bit for bit.
+// A pass of 16,384 rows is one wave of 256 blocks: its time is one block's latency.  Warp w
+// owns rows 16 (w >> 1).. and columns 32 (w & 1).. of every 64 x 64 product, so a layer's
+// SiLU derivatives stay in the registers of the lanes that need them in the backward pass;
+// the fragments, transposed ones too, come by ldmatrix from padded rows; the bias
+// gradients, serial sums over 64 rows, are left for the end, each layer on its own warps.
+// Measured (16,384 rows, one Adam step with its reduction): 95 -> 20 us against single
+// 2-byte fragment loads from unpadded rows.
 __global__ void __launch_bounds__(kTrainThreads, 2) k_mlp_train_tile(const float* __restrict__ params,
                                                                      const bf16* __restrict__ wb,
                                                                      const float* __restrict__ rec, int n, int row0,
                                                                      int row_end, int rows_total,
                                                                      float* __restrict__ part,
                                                                      float* __restrict__ part_loss) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int base = row0 + blockIdx.x * kTrainRows;
     float* const grad = part + (long)blockIdx.x * kNumParams;
-    // the bf16 copy of the weights (refreshed by every Adam step) has the layout of
-    // W1..W4 here: one 16-byte copy per 8 weights; the rows of W1^T repeat their 7
-    // weights in columns 7..13, against the lo halves of the features (mlp_features)
-    static_assert(kNumWeights % 8 == 0 && kOffW2 == 128 * 8, "weight copy in 16-byte pieces");
-    for (int r = tid; r < 64; r += kTrainThreads) {
-        const uint4 a = reinterpret_cast<const uint4*>(wb)[2 * r], b = reinterpret_cast<const uint4*>(wb)[2 * r + 1];
-        const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        const bf16* w = reinterpret_cast<const bf16*>(u);
-        bf16 d[16];
-#pragma unroll
-        for (int k = 0; k < kMlpFeat; ++k) d[k] = d[kMlpFeat + k] = w[k];
-        d[14] = d[15] = __float2bfloat16(0.0f);
-        reinterpret_cast<uint4*>(S.W1 + 16 * r)[0] = reinterpret_cast<const uint4*>(d)[0];
-        reinterpret_cast<uint4*>(S.W1 + 16 * r)[1] = reinterpret_cast<const uint4*>(d)[1];
-    }
-    for (int i = 128 + tid; i < kNumWeights / 8; i += kTrainThreads)
-        reinterpret_cast<uint4*>(S.W1)[i] = reinterpret_cast<const uint4*>(wb)[i];
-    for (int i = tid; i < 200; i += kTrainThreads) S.b[i] = params[kOffB1 + i];
+    // the records do not depend on the previous kernel (the first pass has none)
     for (int r = tid; r < kTrainRows; r += kTrainThreads) {
         const long gi = (long)(base + r) % n;  // wrap around the record set
         const float* q = rec + 8 * gi;
         const bool live = base + r < row_end;
         float ln[3] = {q[0], q[1], q[2]};
-        const float sc = mlp_features(ln, q[3], (int)q[4], S.X + r * 16);
+        const float sc = mlp_features(ln, q[3], (int)q[4], S.X + r * kStrideIn);
         for (int k = 0; k < 3; ++k) S.T[r * 4 + k] = live ? q[5 + k] * sc : 0.0f;
         S.T[r * 4 + 3] = live ? 1.0f : 0.0f;  // row weight
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // the bf16 copy of the weights, refreshed by every Adam step, 16 bytes at a time; the
+    // rows of W1^T repeat their 7 weights in columns 7..13, against the lo halves of the
+    // features (mlp_features)
+    static_assert(kNumWeights % 8 == 0 && kOffW2 == 128 * 8, "weight copy in 16-byte pieces");
+    const uint4* const w16 = reinterpret_cast<const uint4*>(wb);
+    for (int r = tid; r < 64; r += kTrainThreads) {
+        const uint4 a = w16[2 * r], b = w16[2 * r + 1];
+        const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const bf16* w = reinterpret_cast<const bf16*>(u);
+        __align__(16) bf16 d[16];
+#pragma unroll
+        for (int k = 0; k < kMlpFeat; ++k) d[k] = d[kMlpFeat + k] = w[k];
+        d[14] = d[15] = __float2bfloat16(0.0f);
+        reinterpret_cast<uint4*>(S.W1 + kStrideIn * r)[0] = reinterpret_cast<const uint4*>(d)[0];
+        reinterpret_cast<uint4*>(S.W1 + kStrideIn * r)[1] = reinterpret_cast<const uint4*>(d)[1];
+    }
+    for (int i = tid; i < (64 + 64 + 8) * 8; i += kTrainThreads)  // W2, W3, W4: rows of 8 pieces, in sequence
+        *reinterpret_cast<uint4*>(S.W2 + (i >> 3) * kStrideH + (i & 7) * 8) = w16[128 + i];
+    for (int i = tid; i < 200; i += kTrainThreads) S.b[i] = params[kOffB1 + i];
     __syncthreads();
+    const int g = lane >> 2, t = lane & 3;
+    const int m0 = 16 * (warp >> 1), n0 = 32 * (warp & 1);
+    // the lane's entries of tile j: rows m0 + g and m0 + g + 8, columns n0 + 8 j + 2 t, + 1
+    float ds[3][4][4];  // silu' at the pre-activations of the lane's entries
     // ---- forward
-    const bf16* Hin[4] = {S.X, S.H[0], S.H[1], S.H[2]};
-    const bf16* Wl[3] = {S.W1, S.W2, S.W3};
-    const int Kin[3] = {16, 64, 64};
+#pragma unroll
     for (int l = 0; l < 3; ++l) {
-        for (int tt = warp; tt < 32; tt += kTrainWarps) {  // 4 m-tiles x 8 n-tiles
-            const int m0 = (tt >> 3) * 16, n0 = (tt & 7) * 8;
-            float c[4] = {0, 0, 0, 0};
-            if (l == 0) tile_mma<16>(c, Hin[0], 16, 1, kTrainRows, Wl[0], 1, 16, 16, m0, n0, lane);
-            else tile_mma<64>(c, Hin[l], 64, 1, kTrainRows, Wl[l], 1, 64, 64, m0, n0, lane);
-            const int g = lane >> 2, t = lane & 3;
-            for (int e = 0; e < 4; ++e) {
-                const int r = m0 + g + (e >> 1) * 8, col = n0 + 2 * t + (e & 1);
-                const float z = c[e] + S.b[64 * l + col];
-                S.Z[l][r * 64 + col] = z;
-                S.H[l][r * 64 + col] = __float2bfloat16(silu(z));
-            }
+        float c[4][4] = {};
+        if (l == 0) strip_mma<false, false, 16>(c, S.X, kStrideIn, m0, S.W1, kStrideIn, n0, lane);
+        else strip_mma<false, false, 64>(c, S.H[l - 1], kStrideH, m0, l == 1 ? S.W2 : S.W3, kStrideH, n0, lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int col = n0 + 8 * j + 2 * t;
+            const float b0 = S.b[64 * l + col], b1 = S.b[64 * l + col + 1];
+            const float z[4] = {c[j][0] + b0, c[j][1] + b1, c[j][2] + b0, c[j][3] + b1};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ds[l][j][e] = dsilu(z[e]);
+            *reinterpret_cast<uint32_t*>(&S.H[l][(m0 + g) * kStrideH + col]) = pack_bf16x2(silu(z[0]), silu(z[1]));
+            *reinterpret_cast<uint32_t*>(&S.H[l][(m0 + g + 8) * kStrideH + col]) = pack_bf16x2(silu(z[2]), silu(z[3]));
         }
         __syncthreads();
-        (void)Kin;
     }
     if (warp >= 4) {
         if (lane == 0) S.wloss[warp] = 0.0f;
     } else {  // output layer: 4 m-tiles x 1 n-tile, one per warp
-        const int m0 = warp * 16;
+        const int r0 = 16 * warp;
         float c[4] = {0, 0, 0, 0};
-        tile_mma<64>(c, S.H[2], 64, 1, kTrainRows, S.W4, 1, 64, 64, m0, 0, lane);
-        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int k0 = 0; k0 < 64; k0 += 32) {
+            uint32_t a[4], b[4];
+            ldmatrix_x4(S.W4 + (lane & 7) * kStrideH + k0 + 8 * (lane >> 3), b[0], b[1], b[2], b[3]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                ldmatrix_x4(S.H[2] + (r0 + (lane & 15)) * kStrideH + k0 + 16 * h + 8 * (lane >> 4), a[0], a[1], a[2], a[3]);
+                mma_bf16(c, a[0], a[1], a[2], a[3], b[2 * h], b[2 * h + 1]);
+            }
+        }
         float lsum = 0.0f;
+#pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int r = m0 + g + (e >> 1) * 8, col = 2 * t + (e & 1);
+            const int r = r0 + g + (e >> 1) * 8, col = 2 * t + (e & 1);
             const float y = c[e] + S.b[192 + col];
             float d = 0.0f;
             if (col < 3) {
@@ -177,82 +206,93 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_mlp_train_tile(const float
     }
     __syncthreads();
     // ---- backward
-    // dW4t[j][k] = sum_r dY[r][j] H3[r][k]; db4[j] = sum_r dY[r][j]
-    for (int tt = warp; tt < 8; tt += kTrainWarps) {
-        const int n0 = tt * 8;
-        float c[4] = {0, 0, 0, 0};
-        tile_mma<64>(c, S.dY, 1, 8, 8, S.H[2], 64, 1, kTrainRows, 0, n0, lane);
-        const int g = lane >> 2, t = lane & 3;
-        for (int e = 0; e < 4; ++e) {
-            const int j = g + (e >> 1) * 8, k = n0 + 2 * t + (e & 1);
-            if (j < 8) grad[kOffW4 + j * 64 + k] = c[e];
+    // dZ3 = (dY W4^T) * silu'(Z3):  dH3[r][k] = sum_j dY[r][j] W4t[j][k] (8 of 16 k used)
+    {
+        float c[4][4] = {};
+        uint32_t b[4];
+        ldmatrix_x4_t(S.W4 + (lane & 7) * kStrideH + n0 + 8 * (lane >> 3), b[0], b[1], b[2], b[3]);
+        const uint32_t a0 = ld_pair(S.dY + (m0 + g) * 8 + 2 * t), a1 = ld_pair(S.dY + (m0 + g + 8) * 8 + 2 * t);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            mma_bf16(c[j], a0, a1, 0u, 0u, b[j], 0u);
+            const int col = n0 + 8 * j + 2 * t;
+            *reinterpret_cast<uint32_t*>(&S.dZ[2][(m0 + g) * kStrideH + col]) =
+                pack_bf16x2(c[j][0] * ds[2][j][0], c[j][1] * ds[2][j][1]);
+            *reinterpret_cast<uint32_t*>(&S.dZ[2][(m0 + g + 8) * kStrideH + col]) =
+                pack_bf16x2(c[j][2] * ds[2][j][2], c[j][3] * ds[2][j][3]);
         }
     }
-    if (tid < 8) {
-        float s = 0.0f;
-        for (int r = 0; r < kTrainRows; ++r) s += __bfloat162float(S.dY[r * 8 + tid]);
-        grad[kOffB4 + tid] = s;
-    }
-    // dZ3 = (dY W4^T) * silu'(Z3):  dH3[r][k] = sum_j dY[r][j] W4t[j][k]
-    for (int tt = warp; tt < 32; tt += kTrainWarps) {
-        const int m0 = (tt >> 3) * 16, n0 = (tt & 7) * 8;
+    {  // dW4t[j][k] = sum_r dY[r][j] H3[r][k], columns 8 * warp.. (rows j >= 8 of the tile are zero)
         float c[4] = {0, 0, 0, 0};
-        tile_mma<16>(c, S.dY, 8, 1, kTrainRows, S.W4, 64, 1, 8, m0, n0, lane);
-        const int g = lane >> 2, t = lane & 3;
-        for (int e = 0; e < 4; ++e) {
-            const int r = m0 + g + (e >> 1) * 8, k = n0 + 2 * t + (e & 1);
-            S.dZ[0][r * 64 + k] = __float2bfloat16(c[e] * dsilu(S.Z[2][r * 64 + k]));
+#pragma unroll
+        for (int k0 = 0; k0 < kTrainRows; k0 += 32) {
+            uint32_t a[4], b[4];
+            ldmatrix_x4_t(S.dY + (k0 + lane) * 8, a[0], a[1], a[2], a[3]);
+            ldmatrix_x4_t(S.H[2] + (k0 + lane) * kStrideH + 8 * warp, b[0], b[1], b[2], b[3]);
+            mma_bf16(c, a[0], 0u, a[1], 0u, b[0], b[1]);
+            mma_bf16(c, a[2], 0u, a[3], 0u, b[2], b[3]);
         }
+        *reinterpret_cast<float2*>(grad + kOffW4 + g * 64 + 8 * warp + 2 * t) = make_float2(c[0], c[1]);
     }
     __syncthreads();
-    // layers 3, 2, 1: dW_l^T[n][k] = sum_r dZ_l[r][n] H_{l-1}[r][k];  dZ_{l-1} = (dZ_l W_l^T) * silu'
-    const bf16* Wt[3] = {S.W1, S.W2, S.W3};
-    const int offW[3] = {kOffW1, kOffW2, kOffW3};
-    const int offB[3] = {kOffB1, kOffB2, kOffB3};
-    int cur = 0;
-    for (int l = 2; l >= 0; --l) {
-        const bf16* dZ = S.dZ[cur];
-        const bf16* Hp = l == 0 ? S.X : S.H[l - 1];
-        const int kin = l == 0 ? 16 : 64;
-        const int ntiles = (64 / 16) * (kin / 8);
-        for (int tt = warp; tt < ntiles; tt += kTrainWarps) {
-            const int m0 = (tt / (kin / 8)) * 16, n0 = (tt % (kin / 8)) * 8;
-            float c[4] = {0, 0, 0, 0};
-            tile_mma<kTrainRows>(c, dZ, 1, 64, 64, Hp, kin, 1, kTrainRows, m0, n0, lane);
-            const int g = lane >> 2, t = lane & 3;
-            for (int e = 0; e < 4; ++e) {
-                const int nn = m0 + g + (e >> 1) * 8, k = n0 + 2 * t + (e & 1);
-                grad[offW[l] + nn * kin + k] = c[e];
-            }
+    // layers 3, 2: dZ_{l-1} = (dZ_l W_l^T) * silu', then dW_l^T[n][k] = sum_r dZ_l[r][n] H_{l-1}[r][k]
+#pragma unroll
+    for (int l = 2; l > 0; --l) {
+        float c[4][4] = {};
+        strip_mma<false, true, 64>(c, S.dZ[l], kStrideH, m0, l == 1 ? S.W2 : S.W3, kStrideH, n0, lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int col = n0 + 8 * j + 2 * t;
+            *reinterpret_cast<uint32_t*>(&S.dZ[l - 1][(m0 + g) * kStrideH + col]) =
+                pack_bf16x2(c[j][0] * ds[l - 1][j][0], c[j][1] * ds[l - 1][j][1]);
+            *reinterpret_cast<uint32_t*>(&S.dZ[l - 1][(m0 + g + 8) * kStrideH + col]) =
+                pack_bf16x2(c[j][2] * ds[l - 1][j][2], c[j][3] * ds[l - 1][j][3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[j][e] = 0.0f;
         }
-        if (tid < 64) {
-            float s = 0.0f;
-            for (int r = 0; r < kTrainRows; ++r) s += __bfloat162float(dZ[r * 64 + tid]);
-            grad[offB[l] + tid] = s;
-        }
-        if (l > 0) {
-            bf16* dZn = S.dZ[1 - cur];
-            for (int tt = warp; tt < 32; tt += kTrainWarps) {
-                const int m0 = (tt >> 3) * 16, n0 = (tt & 7) * 8;
-                float c[4] = {0, 0, 0, 0};
-                // dH_{l-1}[r][k] = sum_n dZ_l[r][n] W_l^T[n][k]
-                tile_mma<64>(c, dZ, 64, 1, kTrainRows, Wt[l], 64, 1, 64, m0, n0, lane);
-                const int g = lane >> 2, t = lane & 3;
-                for (int e = 0; e < 4; ++e) {
-                    const int r = m0 + g + (e >> 1) * 8, k = n0 + 2 * t + (e & 1);
-                    dZn[r * 64 + k] = __float2bfloat16(c[e] * dsilu(S.Z[l - 1][r * 64 + k]));
-                }
-            }
+        strip_mma<true, true, kTrainRows>(c, S.dZ[l], kStrideH, m0, S.H[l - 1], kStrideH, n0, lane);
+        float* const gw = grad + (l == 1 ? kOffW2 : kOffW3);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = n0 + 8 * j + 2 * t;
+            *reinterpret_cast<float2*>(gw + (m0 + g) * 64 + k) = make_float2(c[j][0], c[j][1]);
+            *reinterpret_cast<float2*>(gw + (m0 + g + 8) * 64 + k) = make_float2(c[j][2], c[j][3]);
         }
         __syncthreads();
-        if (l == 0) {  // W1's gradient: the hi and lo columns of a feature share its weight
-            for (int i = tid; i < 64 * kMlpFeat; i += kTrainThreads) {
-                float* gw = grad + kOffW1 + (i / kMlpFeat) * 16 + i % kMlpFeat;
-                gw[0] += gw[kMlpFeat];
-                gw[kMlpFeat] = 0.0f;
+    }
+    {  // layer 1: one 16x8 tile per warp
+        const int k1 = 8 * (warp & 1);
+        float c[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int k0 = 0; k0 < kTrainRows; k0 += 32) {
+            uint32_t b[4];
+            ldmatrix_x4_t(S.X + (k0 + lane) * kStrideIn + k1, b[0], b[1], b[2], b[3]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t a[4];
+                ldmatrix_x4_t(S.dZ[0] + (k0 + 16 * h + (lane & 7) + 8 * (lane >> 4)) * kStrideH + m0 + 8 * ((lane >> 3) & 1),
+                              a[0], a[1], a[2], a[3]);
+                mma_bf16(c, a[0], a[1], a[2], a[3], b[2 * h], b[2 * h + 1]);
             }
         }
-        cur = 1 - cur;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S.g1[(m0 + g + (e >> 1) * 8) * 17 + k1 + 2 * t + (e & 1)] = c[e];
+    }
+    // bias gradients: the sums over the rows in order
+    if (tid < 200) {
+        const int l = tid >> 6, j = tid & 63, stride = l < 3 ? kStrideH : 8;
+        const bf16* z = (l < 3 ? S.dZ[l] : S.dY) + j;
+        float s = 0.0f;
+#pragma unroll 16
+        for (int r = 0; r < kTrainRows; ++r) s += __bfloat162float(z[r * stride]);
+        grad[kOffB1 + tid] = s;
+    }
+    __syncthreads();
+    // W1's gradient: the hi and lo columns of a feature share its weight
+    for (int i = tid; i < 64 * 16; i += kTrainThreads) {
+        const float* r = S.g1 + (i >> 4) * 17;
+        const int k = i & 15;
+        grad[kOffW1 + i] = k < kMlpFeat ? r[k] + r[kMlpFeat + k] : k < 2 * kMlpFeat ? 0.0f : r[k];
     }
     if (tid == 0) {
         float l = 0.0f;
@@ -261,54 +301,64 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_mlp_train_tile(const float
     }
 }
 
+// Adam (Kingma & Ba 2015) on the f32 master parameters
+struct AdamArgs {
+    float *p, *m, *v;
+    bf16* wb;
+    float lr, b1, b2, eps, c1, c2;
+};
+
 // grad[i] (+)= sum over the blocks of part[b][i]; loss likewise.  A block of 256
 // threads takes 32 parameters: thread (q, i) sums the blocks q*c .. q*c + c - 1 of
 // parameter i in order (c = ceil(blocks / 8)), and the eight partial sums are added
-// in q order, so the result is the same on every run.
+// in q order, so the result is the same on every run.  kAdam (a step's last pass): the
+// parameter, its moments and its bf16 copy are updated here and the gradient is left zero;
+// a launch of its own for that took 3 us of every step.
 constexpr int kReduceParams = 32;
 constexpr int kReduceSplit = 8;
+template <bool kAdam>
 __global__ void __launch_bounds__(kReduceParams * kReduceSplit) k_mlp_reduce(const float* __restrict__ part,
                                                                             const float* __restrict__ part_loss,
                                                                             int blocks, float* __restrict__ grad,
-                                                                            float* __restrict__ loss, int accumulate) {
+                                                                            float* __restrict__ loss, int accumulate,
+                                                                            AdamArgs A) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float ps[kReduceSplit][kReduceParams + 1];
+    __shared__ float pl[kPartBlocks];
     const int ii = threadIdx.x % kReduceParams, q = threadIdx.x / kReduceParams;
     const int i = blockIdx.x * kReduceParams + ii;
     const int c = (blocks + kReduceSplit - 1) / kReduceSplit;
     const int b0 = q * c, b1 = min(blocks, b0 + c);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (blockIdx.x == 0)  // the losses, summed in order below
+        for (int b = threadIdx.x; b < blocks; b += kReduceParams * kReduceSplit) pl[b] = part_loss[b];
     float s = 0.0f;
-    if (i < kNumParams)
+    if (i < kNumParams) {
+#pragma unroll 16
         for (int b = b0; b < b1; ++b) s += part[(long)b * kNumParams + i];
+    }
     ps[q][ii] = s;
     __syncthreads();
     if (q == 0 && i < kNumParams) {
         float t = accumulate ? grad[i] : 0.0f;
 #pragma unroll
         for (int k = 0; k < kReduceSplit; ++k) t += ps[k][ii];
-        grad[i] = t;
+        if (kAdam) {
+            const float mi = A.b1 * A.m[i] + (1.0f - A.b1) * t;
+            const float vi = A.b2 * A.v[i] + (1.0f - A.b2) * t * t;
+            A.m[i] = mi;
+            A.v[i] = vi;
+            const float pi = A.p[i] - A.lr * (mi / A.c1) / (sqrtf(vi / A.c2) + A.eps);
+            A.p[i] = pi;
+            if (i < kNumWeights) A.wb[i] = __float2bfloat16(pi);
+        }
+        grad[i] = kAdam ? 0.0f : t;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == kReduceParams) {
         float l = accumulate ? *loss : 0.0f;
-        for (int b = 0; b < blocks; ++b) l += part_loss[b];
+        for (int b = 0; b < blocks; ++b) l += pl[b];
         *loss = l;
     }
-}
-
-// Adam (Kingma & Ba 2015) on the f32 master parameters; zeroes the gradient and
-// refreshes the bf16 weight copies
-__global__ void k_mlp_adam(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                           bf16* __restrict__ wb, float lr, float b1, float b2, float eps, float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kNumParams) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    p[i] = pi;
-    g[i] = 0.0f;
-    if (i < kNumWeights) wb[i] = __float2bfloat16(pi);
 }
 
 __global__ void k_mlp_refresh_bf16(const float* __restrict__ p, bf16* __restrict__ wb) {
@@ -383,6 +433,24 @@ MlpParams mlp_device_params(const aep_mlp* m) {
         }                                                                       \
     } while (0)
 
+// a launch whose kernel waits for the previous one itself (griddepcontrol.wait), so that
+// its start overlaps that one's end
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_after(void (*kernel)(KArgs...), int grid, int block, size_t smem, bool early, cudaStream_t s,
+                                Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 extern "C" {
 
 aep_status aep_mlp_create(uint64_t seed, aep_mlp** out) {
@@ -453,8 +521,11 @@ aep_status aep_mlp_set_params(aep_mlp* mlp, const float* host, int64_t count) {
 }
 
 // gradient and loss of `rows` records from row0 (cyclic) into mlp->g / mlp->loss:
-// passes of at most kPartBlocks blocks, each reduced in block order
-static aep_status grad_pass(aep_mlp* mlp, const float* rec, int64_t n, int64_t row0, int rows, cudaStream_t s) {
+// passes of at most kPartBlocks blocks, each reduced in block order; adam: the last
+// reduction updates the parameters.  follows: the previous kernel in the stream is a
+// reduction of this network (the records are read before that one has completed)
+static aep_status grad_pass(aep_mlp* mlp, const float* rec, int64_t n, int64_t row0, int rows, cudaStream_t s,
+                            const AdamArgs* adam = nullptr, bool follows = false) {
     static bool attr = false;
     if (!attr) {
         MCK(cudaFuncSetAttribute(k_mlp_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
@@ -463,14 +534,13 @@ static aep_status grad_pass(aep_mlp* mlp, const float* rec, int64_t n, int64_t r
     const int blocks = (rows + kTrainRows - 1) / kTrainRows;
     for (int b0 = 0; b0 < blocks; b0 += kPartBlocks) {
         const int nb = std::min(kPartBlocks, blocks - b0);
-        k_mlp_train_tile<<<nb, kTrainThreads, sizeof(TrainSmem), s>>>(mlp->p, mlp->wb, rec, (int)n,
-                                                                      (int)(row0 + (int64_t)b0 * kTrainRows),
-                                                                      (int)(row0 + rows), rows, mlp->part,
-                                                                      mlp->part_loss);
-        MCK(cudaGetLastError());
-        k_mlp_reduce<<<(kNumParams + kReduceParams - 1) / kReduceParams, kReduceParams * kReduceSplit, 0, s>>>(
-            mlp->part, mlp->part_loss, nb, mlp->g, mlp->loss, b0 > 0 ? 1 : 0);
-        MCK(cudaGetLastError());
+        MCK(launch_after(k_mlp_train_tile, nb, kTrainThreads, sizeof(TrainSmem), follows || b0 > 0, s, mlp->p, mlp->wb,
+                         rec, (int)n, (int)(row0 + (int64_t)b0 * kTrainRows), (int)(row0 + rows), rows, mlp->part,
+                         mlp->part_loss));
+        const bool last = adam && b0 + kPartBlocks >= blocks;
+        MCK(launch_after(last ? k_mlp_reduce<true> : k_mlp_reduce<false>, (kNumParams + kReduceParams - 1) / kReduceParams,
+                         kReduceParams * kReduceSplit, 0, true, s, mlp->part, mlp->part_loss, nb, mlp->g, mlp->loss,
+                         b0 > 0 ? 1 : 0, last ? *adam : AdamArgs{}));
     }
     return AEP_OK;
 }
@@ -501,13 +571,12 @@ aep_status aep_mlp_train(aep_mlp* mlp, const float* d_records, int64_t n, int64_
         const double frac = steps > 1 ? (double)it / (double)(steps - 1) : 1.0;
         const double lri = lr_final + 0.5 * (lr - lr_final) * (1.0 + std::cos(3.14159265358979323846 * frac));
         const bool report = it == steps - 1;
-        aep_status st = grad_pass(mlp, d_records, n, row0 % n, batch, s);
+        const double t = (double)(mlp->t + 1);
+        const float c1 = 1.0f - (float)std::pow(b1, t), c2 = 1.0f - (float)std::pow(b2, t);
+        const AdamArgs adam{mlp->p, mlp->m, mlp->v, mlp->wb, (float)lri, b1, b2, eps, c1, c2};
+        aep_status st = grad_pass(mlp, d_records, n, row0 % n, batch, s, &adam, it > 0);
         if (st) return st;
         ++mlp->t;
-        const float c1 = 1.0f - (float)std::pow(b1, (double)mlp->t), c2 = 1.0f - (float)std::pow(b2, (double)mlp->t);
-        k_mlp_adam<<<(kNumParams + 255) / 256, 256, 0, s>>>(mlp->p, mlp->g, mlp->m, mlp->v, mlp->wb, (float)lri, b1,
-                                                            b2, eps, c1, c2);
-        MCK(cudaGetLastError());
         row0 += batch;
         if (report) {
             float l = 0.f;
