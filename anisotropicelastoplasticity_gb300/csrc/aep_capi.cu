@@ -110,8 +110,10 @@ struct aep_solver {
     int nfixed = 0;
     // adaptive solve loop: device state, its pinned host copy, callback
     SolveState* solve = nullptr;
+    // read back after every step of aep_solve, two steps in flight (pinned, [2])
     SolveState* solve_host = nullptr;
     DevStats* stats_host = nullptr;
+    cudaEvent_t solve_read[2] = {};
     aep_solve_fn solve_fn = nullptr;
     void* solve_user = nullptr;
     int64_t max_steps = 0;
@@ -602,6 +604,8 @@ aep_status aep_solver_destroy(aep_solver* s) {
     cudaFree(s->solve);
     cudaFreeHost(s->solve_host);
     cudaFreeHost(s->stats_host);
+    for (cudaEvent_t e : s->solve_read)
+        if (e) cudaEventDestroy(e);
     for (int r = 0; r < aep_solver::kRing; ++r)
         for (int p = 0; p <= AEP_NUM_PHASES; ++p)
             if (s->ev[r][p]) cudaEventDestroy(s->ev[r][p]);
@@ -1068,8 +1072,9 @@ aep_status aep_solve(aep_solver* s, double cfl, double maxt, double alpha) {
     if (!s->have_particles) return fail(s, AEP_NOT_READY, "aep_solve: no particles");
     if (!s->solve) {
         CK(cudaMalloc(&s->solve, sizeof(SolveState)));
-        CK(cudaMallocHost(&s->solve_host, sizeof(SolveState)));
-        CK(cudaMallocHost(&s->stats_host, sizeof(DevStats)));
+        CK(cudaMallocHost(&s->solve_host, 2 * sizeof(SolveState)));
+        CK(cudaMallocHost(&s->stats_host, 2 * sizeof(DevStats)));
+        for (cudaEvent_t& e : s->solve_read) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     // the first P2G of solve computes densities and volumes (:853-855)
     aep_status st = aep_init_volumes(s);
@@ -1081,28 +1086,50 @@ aep_status aep_solve(aep_solver* s, double cfl, double maxt, double alpha) {
     init.inv_hmin = 1.0 / hmin;
     CK(cudaMemcpyAsync(s->solve, &init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
     s->solve_last = aep_solve_state{};
-    double t = 0.0;
-    int64_t it = 0;
-    while (t <= maxt && (s->max_steps <= 0 || it < s->max_steps)) {
-        st = step_impl(s, 0.0, 0.0, AEP_STAGE_FULL, true);
-        if (st) return st;
-        CK(cudaMemcpyAsync(s->solve_host, s->solve, sizeof(SolveState), cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaMemcpyAsync(s->stats_host, s->dstats, sizeof(DevStats), cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaStreamSynchronize(s->stream));
-        if (s->stats_host->overflow) return fail(s, AEP_OVERFLOW, "fixed-point grid accumulator overflow");
-        const SolveState& h = *s->solve_host;
+    // A step's clock is read back while the next one already runs, where the next one is
+    // certain to follow: no callback may end the solve, and t, which only moves at the end
+    // of a frame, cannot move in the step in flight (Dt <= CFL / 300).  Waiting for every
+    // step before the launch of the next left the device idle between them (131,072
+    // particles, 24 steps and the exchange: 4.12 -> 3.86 ms).  Should the step in flight overflow, the
+    // one after it has run as well; the statistics kept are those of the overflow.
+    double t = 0.0, inner = 0.0;  // after the last step read
+    int64_t launched = 0, read = 0;
+    for (;;) {
+        aep_status launch = AEP_OK;
+        while (launch == AEP_OK && launched - read < 2 && t <= maxt && (s->max_steps <= 0 || launched < s->max_steps) &&
+               (launched == read || (!s->solve_fn && inner + cfl / 3e2 < 1.0 / 60.0))) {
+            launch = step_impl(s, 0.0, 0.0, AEP_STAGE_FULL, true);
+            if (launch) break;
+            const int k = (int)(launched++ & 1);
+            CK(cudaMemcpyAsync(s->solve_host + k, s->solve, sizeof(SolveState), cudaMemcpyDeviceToHost, s->stream));
+            CK(cudaMemcpyAsync(s->stats_host + k, s->dstats, sizeof(DevStats), cudaMemcpyDeviceToHost, s->stream));
+            CK(cudaEventRecord(s->solve_read[k], s->stream));
+        }
+        if (launched == read) return launch;
+        const int k = (int)(read++ & 1);
+        CK(cudaEventSynchronize(s->solve_read[k]));
+        if (s->stats_host[k].overflow) {
+            if (launched > read)
+                CK(cudaMemcpyAsync(s->dstats, s->stats_host + k, sizeof(DevStats), cudaMemcpyHostToDevice, s->stream));
+            CK(cudaStreamSynchronize(s->stream));
+            return fail(s, AEP_OVERFLOW, "fixed-point grid accumulator overflow");
+        }
+        const SolveState& h = s->solve_host[k];
         t = h.t;
-        ++it;
+        inner = h.inner;
         aep_solve_state& o = s->solve_last;
         o.t = h.t;
         o.inner_t = h.inner;
         o.dt = h.Dt;
-        o.steps = it;
+        o.steps = read;
         o.frames = h.frame;
         o.frame_done = h.frame_flag;
-        if (s->solve_fn && s->solve_fn(s, &o, s->solve_user) != 0) break;
+        if (s->solve_fn && s->solve_fn(s, &o, s->solve_user) != 0) return AEP_OK;
+        if (launch) {  // the step after the one read could not be launched
+            CK(cudaStreamSynchronize(s->stream));
+            return launch;
+        }
     }
-    return AEP_OK;
 }
 
 aep_status aep_set_fixed_vertices(aep_solver* s, int64_t nv, const double* vertex_is_fixed) {
