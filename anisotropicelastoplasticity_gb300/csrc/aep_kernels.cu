@@ -54,20 +54,20 @@ __global__ void k_keys(KParams P, PArrays cur, int n, uint32_t* keys, DevStats* 
 // D^-1 = 3/h^2 (:177), x_i - x_p = (o - 1 - f) h  =>  w (b + Mh o) with
 // Mh[:,a] = m D^-1 h_a B[:,a] and b = m v - Mh (1 + f).
 constexpr int kP2GThreads = 128;
-// the P2G grid tile: 3 x 2 x 2 node blocks from the node block of the thread
-// block's first particle (the particles are ordered by node block, x fastest: a
-// block's 512 particles mostly sit in two x-adjacent node blocks, whose stencils
-// the tile holds)
-constexpr int kP2GTileBx = 3;
-constexpr int kP2GTileNodes = kP2GTileBx * 2 * 2 * 64;
+// the P2G grid tile: the 11 x 7 x 7 nodes that hold the stencils based in two x-adjacent
+// node blocks, from the node block of the thread block's first particle (the particles are
+// ordered by node block, x fastest: a block's 512 particles mostly sit there); rows of 12, so
+// that a stencil layer's 16 columns lie on distinct banks
+constexpr int kP2GTileX = 12, kP2GTileY = 7, kP2GTileZ = 7;
+constexpr int kP2GTileNodes = kP2GTileX * kP2GTileY * kP2GTileZ;
 constexpr int kP2GMaxChunk = 128;  // particles per warp at most (the launch picks the chunk)
-// Prep record of one particle, 9 float4 (36 words, 16-byte aligned):
+// Prep record of one particle, 7 float4 (28 words, 16-byte aligned):
 //   q0 = (b, m)  q1 = Mh[0..3]  q2 = Mh[4..7]  q3 = (Mh[8], T lo, T hi, -)
-//   q4 = wx  q5 = wy  q6 = wz  q7 = (base, key)
-// A lane writes its own record with 128-bit stores; a stride of 36 words puts
+//   q4 = wx  q5 = wy  q6 = wz
+// A lane writes its own record with 128-bit stores; a stride of 28 words puts
 // the 8 lanes of each store wavefront on distinct banks; the whole warp then
 // reads one record at a time (broadcast).
-constexpr int kP2GRec = 9;
+constexpr int kP2GRec = 7;
 constexpr int kP2GRegion = 32 * kP2GRec;  // float4 per warp region
 __device__ __forceinline__ void mark_blocks(const KParams& P, const GArrays& G, uint32_t key) {
     uint32_t blk = key >> 6;
@@ -93,12 +93,15 @@ __device__ __forceinline__ void mark_blocks(const KParams& P, const GArrays& G, 
 // t + h, t + h + 2, ..., accumulating the column's 4 nodes x (mass, momentum) in
 // FP32 registers.  At the end of a run (warp-uniform) the halves' sums are added,
 // half h takes the z-layers 2h, 2h + 1, and the node sums are rounded to fixed
-// point and added as integers: runs whose stencil lies in the block's grid tile
-// (3 x 2 x 2 node blocks from the node block of its first particle, which holds the
-// stencils of that node block's particles and of the next one's in x: ~91% of the
-// runs on the sand + cloth scene, against ~68% for the 2 x 2 x 2 blocks of the
-// middle particle) into a fixed-point copy of the tile in shared memory, which is
-// added to the grid once per node at the end; other runs into the grid directly.
+// point and added as integers: runs whose stencil lies in the block's grid tile (the
+// nodes of the stencils based in the node block of its first particle and in the next one
+// in x: ~91% of the runs on the sand + cloth scene) into a fixed-point copy of the tile in
+// shared memory, which is added to the grid once per node at the end; other runs into the
+// grid directly.  The kernel waits for shared memory and shuffles (2.3 of 7 stalls per
+// issue), so warps count: with only those nodes in the tile (588 against the 768 of 3 x 2 x 2
+// whole node blocks) and records of 28 words, 24 warps fit an SM instead of 20.  Measured:
+// 929 -> 842 us for 8,388,608 particles at 512^3, 277 -> 254 for 2,097,152 at 256^3, 46.6 for
+// 100,003 at 64^3 as before (a base decoded from the key in place of shuffled: 829, 252, 49.4).
 // Integer sums: the result does not depend on the order.
 // A small system (share > 0) gives a batch of 32 particles to two or four warps, which all
 // prepare it and take its runs in turn: its time is the latency of one warp's runs (4.7 of
@@ -113,7 +116,7 @@ __device__ __forceinline__ void mark_blocks(const KParams& P, const GArrays& G, 
 // bit from step to step.  T - S is far below 2^31 (FP32 weight-sum error and
 // roundings), so it is computed from the low 32 bits of T and of the node masses
 // with one 32-bit warp reduction.
-__global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, const uint32_t* __restrict__ keys,
+__global__ void __launch_bounds__(kP2GThreads, 6) k_p2g(KParams P, PArrays cur, const uint32_t* __restrict__ keys,
                                                      const int32_t* __restrict__ perm, int n, int chunk, int share,
                                                      GArrays G, int32_t* __restrict__ slot_of,
                                                      int32_t* __restrict__ curidx_of) {
@@ -132,51 +135,41 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
     const unsigned mine = share ? ((1u << part) - 1u) << part0 : 0xffffffffu;
     const int cnt_total = (int)max(0L, min((long)chunk, (long)n - chunk0));  // warp-uniform
     // the tile's origin: the node block of the block's first particle
-    int org[3];
-    tile_origin(P, keys[min(blk0, (long)n - 1)], org);
+    const uint32_t oblk = keys[min(blk0, (long)n - 1)] >> 6;
+    const uint32_t last_x = oblk % (uint32_t)P.nb[0] == (uint32_t)P.nb[0] - 1u ? 1u : 2u;  // its node blocks in x
     for (int i = threadIdx.x; i < 4 * kP2GTileNodes; i += kP2GThreads) tacc[i] = 0ull;
     __syncthreads();
 
     float am[4] = {0, 0, 0, 0}, ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0}, az[4] = {0, 0, 0, 0};
     uint32_t run_key = kInvalidKey;
-    int rb[3] = {0, 0, 0};
+    int rb[3] = {0, 0, 0};  // the run's padded base node
     long long run_T = 0;
     auto flush = [&]() {  // warp-uniform
         if (run_key == kInvalidKey) return;
-        // the two halves' sums added; half h then adds z-layers 2h, 2h + 1
-#pragma unroll
-        for (int oz = 0; oz < 4; ++oz) {
-            am[oz] += __shfl_xor_sync(0xffffffffu, am[oz], 16);
-            ax[oz] += __shfl_xor_sync(0xffffffffu, ax[oz], 16);
-            ay[oz] += __shfl_xor_sync(0xffffffffu, ay[oz], 16);
-            az[oz] += __shfl_xor_sync(0xffffffffu, az[oz], 16);
-        }
-        run_T += __shfl_xor_sync(0xffffffffu, run_T, 16);
+        // the two halves' sums added: half h keeps z-layers 2h, 2h + 1 and gives the others
         float gm[2], gx[2], gy[2], gz[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            gm[k] = half ? am[2 + k] : am[k];
-            gx[k] = half ? ax[2 + k] : ax[k];
-            gy[k] = half ? ay[2 + k] : ay[k];
-            gz[k] = half ? az[2 + k] : az[k];
+            gm[k] = (half ? am[2 + k] : am[k]) + __shfl_xor_sync(0xffffffffu, half ? am[k] : am[2 + k], 16);
+            gx[k] = (half ? ax[2 + k] : ax[k]) + __shfl_xor_sync(0xffffffffu, half ? ax[k] : ax[2 + k], 16);
+            gy[k] = (half ? ay[2 + k] : ay[k]) + __shfl_xor_sync(0xffffffffu, half ? ay[k] : ay[2 + k], 16);
+            gz[k] = (half ? az[2 + k] : az[k]) + __shfl_xor_sync(0xffffffffu, half ? az[k] : az[2 + k], 16);
         }
+        run_T += __shfl_xor_sync(0xffffffffu, run_T, 16);
         long long mf[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) mf[k] = __float2ll_rn(gm[k] * P.mass_scale);
         const unsigned s_lo = __reduce_add_sync(0xffffffffu, (unsigned)mf[0] + (unsigned)mf[1]);
         if (lane == 5) mf[1] += (long long)(int)((unsigned)run_T - s_lo);  // (ox, oy, oz) = (1, 1, 1)
-        const int x = rb[0] + ox, y = rb[1] + oy;
-        const int rbx = (rb[0] >> 2) - org[0];
-        if (rbx >= 0 && rbx < kP2GTileBx - 1 && (rb[1] >> 2) == org[1] && (rb[2] >> 2) == org[2]) {
-            // the run's stencil (base .. base + 3) lies in the tile: node blocks
-            // org.x + rbx, org.x + rbx + 1 in x, org.y, org.y + 1, org.z, org.z + 1
-            const int tx = x - 4 * org[0], ty = y - 4 * org[1];
-            const int txy = (tx >> 2) * 64 + (tx & 3) + (ty >> 2) * (64 * kP2GTileBx) + ((ty & 3) << 2);
+        const uint32_t d = (run_key >> 6) - oblk;
+        if (d < last_x) {
+            // the run's stencil (base .. base + 3) lies in the tile
+            const int tx = 4 * (int)d + (int)(run_key & 3u) + ox, ty = (int)((run_key >> 2) & 3u) + oy;
+            const int tz = (int)((run_key >> 4) & 3u) + 2 * half;
+            unsigned long long* a = tacc + (tz * kP2GTileY + ty) * kP2GTileX + tx;
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
+            for (int k = 0; k < 2; ++k, a += kP2GTileX * kP2GTileY) {
                 if (mf[k] != 0) {
-                    const int tz = rb[2] + 2 * half + k - 4 * org[2];
-                    unsigned long long* a = tacc + txy + (tz >> 2) * (128 * kP2GTileBx) + ((tz & 3) << 4);
                     atomicAdd(a, (unsigned long long)mf[k]);
                     atomicAdd(a + kP2GTileNodes, to_fixed(gx[k], P.mom_scale));
                     atomicAdd(a + 2 * kP2GTileNodes, to_fixed(gy[k], P.mom_scale));
@@ -187,7 +180,7 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 if (mf[k] != 0) {
-                    unsigned long long* a = acc_node(G, node_index(P, x, y, rb[2] + 2 * half + k));
+                    unsigned long long* a = acc_node(G, node_index(P, rb[0] + ox, rb[1] + oy, rb[2] + 2 * half + k));
                     atomicAdd(a, (unsigned long long)mf[k]);
                     atomicAdd(a + kAccX, to_fixed(gx[k], P.mom_scale));
                     atomicAdd(a + kAccY, to_fixed(gy[k], P.mom_scale));
@@ -203,6 +196,7 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
     for (int b0 = 0; b0 < cnt_total; b0 += 32) {
         const long j = chunk0 + b0 + lane;
         uint32_t my_key = kInvalidKey;
+        int base[3] = {0, 0, 0};
         const int pj_cur = b0 + lane < cnt_total ? perm[j] : 0;
         float xs_[16];  // the batch's particle state: x, m, v, B
 #pragma unroll
@@ -228,6 +222,8 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
             int cell[3];
             float f[3], w[3][4], dw[3][4];
             locate(P, xp[0], xp[1], xp[2], cell, f);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) base[a] = cell[a] + 3;
             const bool trunc = particle_weights(P, cell, f, w, dw);
             // exact fixed-point mass; a stencil cut by the grid boundary keeps only
             // the weight inside the grid (HS:44-46), as the reference does
@@ -257,8 +253,6 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
             r[4] = make_float4(w[0][0], w[0][1], w[0][2], w[0][3]);
             r[5] = make_float4(w[1][0], w[1][1], w[1][2], w[1][3]);
             r[6] = make_float4(w[2][0], w[2][1], w[2][2], w[2][3]);
-            r[7] = make_float4(__int_as_float(cell[0] + 3), __int_as_float(cell[1] + 3), __int_as_float(cell[2] + 3),
-                               __uint_as_float(key));
             my_key = key;
         }
         // run heads: a particle whose key differs from the previous one's (any order)
@@ -271,9 +265,9 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
         for (int t = !share ? 0 : own ? __ffs(own) - 1 : 32; t < cnt && ((mine >> t) & 1u);) {
             if ((heads >> t) & 1u) {
                 flush();
-                const float4 q7 = region[t * kP2GRec + 7];
-                run_key = __float_as_uint(q7.w);
-                rb[0] = __float_as_int(q7.x); rb[1] = __float_as_int(q7.y); rb[2] = __float_as_int(q7.z);
+                run_key = __shfl_sync(0xffffffffu, my_key, t);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) rb[a] = __shfl_sync(0xffffffffu, base[a], t);
             }
             const unsigned after = heads & ~((2u << t) - 1u);  // heads after t (none for t = 31)
             const int e = min(cnt, after ? __ffs(after) - 1 : 32);
@@ -310,17 +304,18 @@ __global__ void __launch_bounds__(kP2GThreads) k_p2g(KParams P, PArrays cur, con
     flush();
     __syncthreads();
     // the tile into the grid, one atomic per nonzero node and channel
+    int org[3];
+    tile_origin(P, oblk << 6, org);
     for (int i = threadIdx.x; i < kP2GTileNodes; i += kP2GThreads) {
-        const int t = i >> 6;  // tile block (bx, by, bz) = (t % 3, (t / 3) % 2, t / 6)
-        const int bx = t % kP2GTileBx, by = (t / kP2GTileBx) & 1, bz = t / (2 * kP2GTileBx);
-        if (org[0] + bx >= P.nb[0]) continue;  // past the padded grid: nothing was added there
-        const uint32_t gblk = (uint32_t)(((org[2] + bz) * P.nb[1] + org[1] + by) * P.nb[0] + org[0] + bx);
-        unsigned long long* a = acc_node(G, (gblk << 6) | (uint32_t)(i & 63));
+        const unsigned long long v[4] = {tacc[i], tacc[kP2GTileNodes + i], tacc[2 * kP2GTileNodes + i],
+                                         tacc[3 * kP2GTileNodes + i]};
+        if ((v[0] | v[1] | v[2] | v[3]) == 0ull) continue;
+        const int r = i / kP2GTileX;
+        unsigned long long* a = acc_node(G, node_index(P, 4 * org[0] + i % kP2GTileX, 4 * org[1] + r % kP2GTileY,
+                                                       4 * org[2] + r / kP2GTileY));
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const unsigned long long v = tacc[c * kP2GTileNodes + i];
-            if (v != 0ull) atomicAdd(a + c * kAccX, v);
-        }
+        for (int c = 0; c < 4; ++c)
+            if (v[c] != 0ull) atomicAdd(a + c * kAccX, v[c]);
     }
 }
 
@@ -2447,13 +2442,13 @@ void launch_p2g(const KParams& P, const PArrays& cur, const uint32_t* keys, cons
                 const GArrays& G, int32_t* slot_of, int32_t* curidx_of, cudaStream_t s) {
     // particles per warp: the particles spread evenly over the fewest waves of the
     // device's resident warps with at most kP2GMaxChunk each, rounded up to a
-    // multiple of 32 (whole batches)
-    static const long slots = [] {  // resident warps of k_p2g on the device
-        int dev = 0, sms = 0, per = 0;
+    // multiple of 32 (whole batches).  The chunk decides where runs are cut and with that
+    // how sums round, so the 20 warps per SM stay (24 are resident)
+    static const long slots = [] {
+        int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_p2g, kP2GThreads, 0);
-        return (long)std::max(1, sms * per) * (kP2GThreads / 32);
+        return (long)std::max(1, sms) * 20;
     }();
     const long waves = std::max(1L, ((long)n + slots * kP2GMaxChunk - 1) / (slots * kP2GMaxChunk));
     const long per_warp = ((long)n + waves * slots - 1) / (waves * slots);
