@@ -424,6 +424,20 @@ constexpr int kFrcRec = 11;
 constexpr int kFrcWarpBuf = 32 * kFrcRec + 1;
 __device__ __forceinline__ int frc_slot(int p) { return p * kFrcRec + (p >= 16 ? 1 : 0); }
 
+// two FP32 FMAs in one instruction (each rounded as fmaf): the rate of two, one issue slot.
+// Measured: the force's scatter with them and with the halves exchanging sums 1,338 -> 1,322 us
+// at 8,388,608 particles, G2P's rows 1,148 -> 1,104; the force's gradient gather got slower
+// (1,376: the weights' copies spill).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+          "l"(reinterpret_cast<const unsigned long long&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+
 // Velocity gradient of the P2G velocity (the three SpMVs of HS:269-271), contracted one
 // axis at a time: Gm = sum v (grad w)^T with grad w = (dwx wy wz, wx dwy wz, wx wy dwz)
 __device__ __forceinline__ void gradient_row(const float4 v[4], const float wx[4], const float dx[4], float cz, float dz,
@@ -718,7 +732,7 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
     // z-layers 2h, 2h + 1 to the grid
     const int h = lane >> 4, l = lane & 15, ox = l & 3, oy = l >> 2;
     const int cnt = (int)max(0l, min(32l, (long)n - chunk0));
-    float fx[4] = {0, 0, 0, 0}, fy[4] = {0, 0, 0, 0}, fz[4] = {0, 0, 0, 0};
+    float2 fx[2] = {}, fy[2] = {}, fz[2] = {};  // two z-layers each
     // run heads: a particle whose key differs from the previous one's (any order)
     const uint32_t key_before = __shfl_up_sync(0xffffffffu, my_key, 1);
     const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || my_key != key_before);
@@ -740,35 +754,35 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
             const float p1 = dxo * wyo, p2 = wxo * dyo, p3 = wxo * wyo;
             const float ax_ = p1 * q0.x + p2 * q0.y, ay_ = p1 * q0.w + p2 * q1.x, az_ = p1 * q1.z + p2 * q1.w;
             const float cx = p3 * q0.z, cy = p3 * q1.y, cz = p3 * q2.x;
-            const float wz4[4] = {q5.x, q5.y, q5.z, q5.w}, dz4[4] = {q8.x, q8.y, q8.z, q8.w};
+            const float2 wz2[2] = {{q5.x, q5.y}, {q5.z, q5.w}}, dz2[2] = {{q8.x, q8.y}, {q8.z, q8.w}};
 #pragma unroll
-            for (int oz = 0; oz < 4; ++oz) {
-                fx[oz] = fmaf(wz4[oz], ax_, fmaf(dz4[oz], cx, fx[oz]));
-                fy[oz] = fmaf(wz4[oz], ay_, fmaf(dz4[oz], cy, fy[oz]));
-                fz[oz] = fmaf(wz4[oz], az_, fmaf(dz4[oz], cz, fz[oz]));
+            for (int k = 0; k < 2; ++k) {
+                fx[k] = fma2(wz2[k], both(ax_), fma2(dz2[k], both(cx), fx[k]));
+                fy[k] = fma2(wz2[k], both(ay_), fma2(dz2[k], both(cy), fy[k]));
+                fz[k] = fma2(wz2[k], both(az_), fma2(dz2[k], both(cz), fz[k]));
             }
             const float4 q10 = r[10];
             if (q10.w != 0.0f) {  // cloth vertex: + w f_v
                 const float wx_ = p3 * q10.x, wy_ = p3 * q10.y, wz_ = p3 * q10.z;
 #pragma unroll
-                for (int oz = 0; oz < 4; ++oz) {
-                    fx[oz] = fmaf(wz4[oz], wx_, fx[oz]);
-                    fy[oz] = fmaf(wz4[oz], wy_, fy[oz]);
-                    fz[oz] = fmaf(wz4[oz], wz_, fz[oz]);
+                for (int k = 0; k < 2; ++k) {
+                    fx[k] = fma2(wz2[k], both(wx_), fx[k]);
+                    fy[k] = fma2(wz2[k], both(wy_), fy[k]);
+                    fz[k] = fma2(wz2[k], both(wz_), fz[k]);
                 }
             }
         }
         // the run's sums: the two halves added, then z-layers 2h, 2h + 1 from half h
-#pragma unroll
-        for (int oz = 0; oz < 4; ++oz) {
-            fx[oz] += __shfl_xor_sync(0xffffffffu, fx[oz], 16);
-            fy[oz] += __shfl_xor_sync(0xffffffffu, fy[oz], 16);
-            fz[oz] += __shfl_xor_sync(0xffffffffu, fz[oz], 16);
-        }
+        auto fold = [&](const float2 f[2]) {
+            const float2 keep = h ? f[1] : f[0], give = h ? f[0] : f[1];
+            return make_float2(keep.x + __shfl_xor_sync(0xffffffffu, give.x, 16),
+                               keep.y + __shfl_xor_sync(0xffffffffu, give.y, 16));
+        };
+        const float2 sx = fold(fx), sy = fold(fy), sz = fold(fz);
         const int x = rb[0] + ox, y = rb[1] + oy;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            const float gx = h ? fx[2 + k] : fx[k], gy = h ? fy[2 + k] : fy[k], gz = h ? fz[2 + k] : fz[k];
+            const float gx = k ? sx.y : sx.x, gy = k ? sy.y : sy.x, gz = k ? sz.y : sz.x;
             if (gx != 0.0f || gy != 0.0f || gz != 0.0f) {
                 unsigned long long* a = acc_node(G, node_index(P, x, y, rb[2] + 2 * h + k));
                 atomicAdd(a + kAccX, to_fixed(gx, P.mom_scale));
@@ -777,7 +791,7 @@ __global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur
             }
         }
 #pragma unroll
-        for (int oz = 0; oz < 4; ++oz) fx[oz] = fy[oz] = fz[oz] = 0.0f;
+        for (int k = 0; k < 2; ++k) fx[k] = fy[k] = fz[k] = make_float2(0.0f, 0.0f);
         t = e;
     }
 }
@@ -1167,14 +1181,30 @@ struct Gathered {
     float vp[3], C[9], Gb[9];
 };
 // one z row of four nodes, added to the row sums B (weights wx, wxi, dwx; cz, czx, dz)
+template <bool kPacked>
 __device__ __forceinline__ void gather_row(const float4 v[4], const float wx[4], const float wxi[4], const float dx[4],
                                            float cz, float czx, float dz, float B[5][3]) {
     float A0[3] = {0, 0, 0}, A1[3] = {0, 0, 0}, A2[3] = {0, 0, 0};
+    if (kPacked) {  // x and y in one instruction (not in the small form: registers)
+        float2 p0 = {0, 0}, p1 = {0, 0}, p2 = {0, 0};
 #pragma unroll
-    for (int o = 0; o < 4; ++o) {
-        A0[0] = fmaf(wx[o], v[o].x, A0[0]); A0[1] = fmaf(wx[o], v[o].y, A0[1]); A0[2] = fmaf(wx[o], v[o].z, A0[2]);
-        A1[0] = fmaf(wxi[o], v[o].x, A1[0]); A1[1] = fmaf(wxi[o], v[o].y, A1[1]); A1[2] = fmaf(wxi[o], v[o].z, A1[2]);
-        A2[0] = fmaf(dx[o], v[o].x, A2[0]); A2[1] = fmaf(dx[o], v[o].y, A2[1]); A2[2] = fmaf(dx[o], v[o].z, A2[2]);
+        for (int o = 0; o < 4; ++o) {
+            const float2 xy = make_float2(v[o].x, v[o].y);
+            p0 = fma2(both(wx[o]), xy, p0);
+            p1 = fma2(both(wxi[o]), xy, p1);
+            p2 = fma2(both(dx[o]), xy, p2);
+            A0[2] = fmaf(wx[o], v[o].z, A0[2]);
+            A1[2] = fmaf(wxi[o], v[o].z, A1[2]);
+            A2[2] = fmaf(dx[o], v[o].z, A2[2]);
+        }
+        A0[0] = p0.x; A0[1] = p0.y; A1[0] = p1.x; A1[1] = p1.y; A2[0] = p2.x; A2[1] = p2.y;
+    } else {
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+            A0[0] = fmaf(wx[o], v[o].x, A0[0]); A0[1] = fmaf(wx[o], v[o].y, A0[1]); A0[2] = fmaf(wx[o], v[o].z, A0[2]);
+            A1[0] = fmaf(wxi[o], v[o].x, A1[0]); A1[1] = fmaf(wxi[o], v[o].y, A1[1]); A1[2] = fmaf(wxi[o], v[o].z, A1[2]);
+            A2[0] = fmaf(dx[o], v[o].x, A2[0]); A2[1] = fmaf(dx[o], v[o].y, A2[1]); A2[2] = fmaf(dx[o], v[o].z, A2[2]);
+        }
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1210,6 +1240,7 @@ __device__ __forceinline__ void gather_zero(Gathered& g) {
 // of both fields where no flag says that they differ, and cloth elements in the same pass:
 // G2P 92 -> 83 us for 524,288 sand particles at 128^3, 361 -> 299 for 2,097,152 of snow and
 // sand at 256^3, 1,448 -> 1,136 for 8,388,608 with cloth at 512^3.
+template <bool kPacked>
 __device__ __forceinline__ void gather_tile(const float4* t, const float w[3][4], const float dw[3][4],
                                             const float xi[3][4], Gathered& g) {
     float wxi[4], wy[4], wyx[4], dy[4];
@@ -1228,7 +1259,7 @@ __device__ __forceinline__ void gather_tile(const float4* t, const float w[3][4]
         for (int oz = 0; oz < 4; ++oz) {
             const float4 v[4] = {t[oz * kGtX * kGtY], t[oz * kGtX * kGtY + 1], t[oz * kGtX * kGtY + 2],
                                  t[oz * kGtX * kGtY + 3]};
-            gather_row(v, w[0], wxi, dw[0], w[2][oz], w[2][oz] * xi[2][oz], dw[2][oz], B);
+            gather_row<kPacked>(v, w[0], wxi, dw[0], w[2][oz], w[2][oz] * xi[2][oz], dw[2][oz], B);
         }
         gather_add(B, wy[0], wyx[0], dy[0], g);
         t += kGtX;
@@ -1258,7 +1289,7 @@ __device__ __forceinline__ void gather_grid(const KParams& P, const float4* __re
 #pragma unroll
             for (int o = 0; o < 4; ++o) v[o] = f[node_index(P, base[0] + o, base[1] + oy, base[2] + oz)];
             const float cz = pick4(w[2], oz);
-            gather_row(v, w[0], wxi, dw[0], cz, cz * pick4(xi[2], oz), pick4(dw[2], oz), B);
+            gather_row<false>(v, w[0], wxi, dw[0], cz, cz * pick4(xi[2], oz), pick4(dw[2], oz), B);
         }
         const float cy = pick4(w[1], oy);
         gather_add(B, cy, cy * pick4(xi[1], oy), pick4(dw[1], oy), g);
@@ -1384,7 +1415,7 @@ __global__ void __launch_bounds__(128, kSmall || !kDefer ? 4 : 5) k_g2p(KParams 
     float vp[3], xs[3], C[9], Gb[9];
     if (live) {
         Gathered g;
-        if (in_tile || in_tile2) gather_tile(stencil, w, dw, xi, g);
+        if (in_tile || in_tile2) gather_tile<!kSmall>(stencil, w, dw, xi, g);
         else gather_grid(P, G.vel, base, w, dw, xi, g);
 #pragma unroll
         for (int c = 0; c < 3; ++c) vp[c] = xs[c] = g.vp[c];
@@ -1402,7 +1433,7 @@ __global__ void __launch_bounds__(128, kSmall || !kDefer ? 4 : 5) k_g2p(KParams 
     dt = step_dt(P, dt, 1);
     if (in_tile ? two && stencil_differs(base, org, sdiff) : grid_differs(P, base, G.vdiff)) {
         Gathered g;
-        if (vbf2 && in_tile) gather_tile(tile2 + toff, w, dw, xi, g);
+        if (vbf2 && in_tile) gather_tile<false>(tile2 + toff, w, dw, xi, g);
         else gather_grid(P, G.vbf, base, w, dw, xi, g);
 #pragma unroll
         for (int c = 0; c < 3; ++c) xs[c] = g.vp[c];
