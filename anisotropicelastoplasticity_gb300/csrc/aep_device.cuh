@@ -299,22 +299,34 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-// one node of the tile into shared memory (nothing outside the padded grid)
-__device__ __forceinline__ void load_gather_node(const KParams& P, const int org[3], const float4* __restrict__ src,
-                                                 float4* dst, int x, int y, int z) {
-    const int gx = 4 * org[0] - 1 + x, gy = 4 * org[1] - 1 + y, gz = 4 * org[2] - 1 + z;
-    if (gx >= 0 && gy >= 0 && gz >= 0 && gx < 4 * P.nb[0] && gy < 4 * P.nb[1] && gz < 4 * P.nb[2])
-        cp_async16(dst + (z * kGtY + y) * kGtX + x, src + node_index(P, gx, gy, gz));
-}
-// cooperative asynchronous copy of the tile by 128 threads (the caller waits for its
-// copies and synchronises): rows y < 8 of every z by 16 threads each, then the rows y = 8
+// cooperative asynchronous copy of the tile by 128 threads (the caller waits for its copies
+// and synchronises; nothing is copied from outside the padded grid): rows y < 8 of every z by
+// 16 threads each, then the rows y = 8.  A column's nodes along z lie 16 nodes apart inside
+// each of three node blocks, so a copy costs one instruction with a constant offset (with
+// a node index for each: force 1,314 -> 1,297 us, G2P 1,104 -> 1,099 at 8,388,608 particles).
 __device__ __forceinline__ void load_gather_tile(const KParams& P, const int org[3], const float4* __restrict__ src,
                                                  float4* dst) {
-    const int x = threadIdx.x & 15, y = threadIdx.x >> 4;
-    if (x < kGtX)
-#pragma unroll 3
-        for (int z = 0; z < kGtZ; ++z) load_gather_node(P, org, src, dst, x, y, z);
-    if (threadIdx.x < kGtX * kGtZ) load_gather_node(P, org, src, dst, threadIdx.x % kGtX, 8, threadIdx.x / kGtX);
+    {
+        const int x = threadIdx.x & 15, y = threadIdx.x >> 4;
+        const int gx = 4 * org[0] - 1 + x, gy = 4 * org[1] - 1 + y;
+        if (x < kGtX && gx >= 0 && gy >= 0 && gx < 4 * P.nb[0] && gy < 4 * P.nb[1]) {
+            const long zb = 64l * P.nb[0] * P.nb[1];  // nodes from a node block to the next one in z
+            const float4* s = src + node_index(P, gx, gy, 4 * org[2]);
+            float4* d = dst + y * kGtX + x;
+            if (org[2] > 0) cp_async16(d, s - zb + 48);
+#pragma unroll
+            for (int z = 0; z < 4; ++z) cp_async16(d + (z + 1) * kGtX * kGtY, s + 16 * z);
+            if (org[2] + 1 < P.nb[2])
+#pragma unroll
+                for (int z = 0; z < 4; ++z) cp_async16(d + (z + 5) * kGtX * kGtY, s + zb + 16 * z);
+        }
+    }
+    if (threadIdx.x < kGtX * kGtZ) {
+        const int x = threadIdx.x % kGtX, z = threadIdx.x / kGtX;
+        const int gx = 4 * org[0] - 1 + x, gy = 4 * org[1] + 7, gz = 4 * org[2] - 1 + z;
+        if (gx >= 0 && gz >= 0 && gx < 4 * P.nb[0] && gy < 4 * P.nb[1] && gz < 4 * P.nb[2])
+            cp_async16(dst + (z * kGtY + 8) * kGtX + x, src + node_index(P, gx, gy, gz));
+    }
 }
 // whether the stencil from padded node `base` lies in the tile; its offset there
 __device__ __forceinline__ bool gather_offset(const int base[3], const int org[3], int& off) {
