@@ -410,6 +410,23 @@ aep_status download(aep_solver* s, double* dst, int count, int mode, float* cons
 // 32-byte sector.
 constexpr int kRecordValues = 12;
 
+// whether mesh state goes by way of records: every array given is device memory, and a
+// vertex or an element has that many values
+template <typename T>
+bool mesh_by_records(const MeshFields<T>& m) {
+    const T* const all[7] = {m.xv, m.vv, m.Bv, m.xe, m.ve, m.Be, m.d};
+    const int cnt[7] = {3, 3, 9, 3, 3, 9, 9};
+    int values[2] = {0, 0};
+    for (int f = 0; f < 7; ++f)
+        if (all[f]) {
+            bool on_device = false;
+            device_alias(all[f], &on_device);
+            if (!on_device) return false;
+            values[f >= 3] += cnt[f];
+        }
+    return std::max(values[0], values[1]) >= kRecordValues;
+}
+
 aep_status check_overflow(aep_solver* s) {
     DevStats h;
     CK(cudaMemcpy(&h, s->dstats, sizeof(h), cudaMemcpyDeviceToHost));
@@ -843,6 +860,13 @@ aep_status aep_get_mesh(aep_solver* s, double* xv, double* vv, double* Bv, doubl
     PArrays& P = s->P[s->cur];
     const int64_t vb = s->np, eb = s->np + s->nv, ee = s->n;
     const size_t V = (size_t)s->nv, F = (size_t)s->nf;
+    const MeshFields<double> m{(int)s->nv, (int)s->nf, xv, vv, Bv, xe, ve, Be, d};
+    if (mesh_by_records(m)) {
+        launch_download_mesh((int)s->n, (int)vb, m, P, s->staging, s->stream);
+        CKLAUNCH();
+        CK(cudaStreamSynchronize(s->stream));
+        return AEP_OK;
+    }
     aep_status st = prepare_download(s);
     if (st) return st;
     if (xv && (st = download(s, xv, 3, 0, P.x, vb, eb, 0, false))) return st;
@@ -868,6 +892,14 @@ aep_status aep_set_mesh_state(aep_solver* s, int64_t nv, int64_t nf, const doubl
     PArrays& P = s->P[s->cur];
     const int64_t vb = s->np, eb = s->np + s->nv;
     const size_t V = (size_t)s->nv, F = (size_t)s->nf;
+    if (xv || xe) s->keys_valid = false;  // positions changed: fresh keys at the next step
+    const MeshFields<const double> m{(int)nv, (int)nf, xv, vv, Bv, xe, ve, Be, d};
+    if (mesh_by_records(m)) {
+        launch_upload_mesh((int)s->n, (int)vb, m, P, s->staging, s->stream);
+        CKLAUNCH();
+        CK(cudaStreamSynchronize(s->stream));
+        return AEP_OK;
+    }
     launch_inverse_ids((int)s->n, P.id, s->perm, s->stream);  // perm[id] = slot
     CKLAUNCH();
     const int32_t* mv = s->perm + vb;
@@ -881,7 +913,6 @@ aep_status aep_set_mesh_state(aep_solver* s, int64_t nv, int64_t nf, const doubl
     if (ve && (st = upload(s, ve, 3, 0, P.v, nf, 0, me, 15 * V + 3 * F))) return st;
     if (Be && (st = upload(s, Be, 9, 1, P.B, nf, 0, me, 15 * V + 6 * F))) return st;
     if (d && (st = upload(s, d, 9, 4, P.F, nf, 0, me, 15 * V + 15 * F))) return st;
-    if (xv || xe) s->keys_valid = false;  // positions changed: fresh keys at the next step
     CK(cudaStreamSynchronize(s->stream));
     return AEP_OK;
 }

@@ -40,6 +40,15 @@ struct UploadSrc {
 struct DownloadDst {
     double *x, *v, *B, *Fe, *Fp, *vol, *plastic;
 };
+// the mesh state's arrays (LagrangianMesh's layouts; any may be null)
+template <typename T>
+struct MeshFields {
+    int nv, nf;
+    T *xv, *vv, *Bv, *xe, *ve, *Be, *d;
+};
+void launch_upload_mesh(int slots, int id0, const MeshFields<const double>& m, const PArrays& P, void* rec,
+                        cudaStream_t s);
+void launch_download_mesh(int slots, int id0, const MeshFields<double>& m, const PArrays& P, void* rec, cudaStream_t s);
 void launch_upload_particles(int n, const UploadSrc& src, const PArrays& P, const int32_t* map, int track_fp,
                              unsigned long long* check, cudaStream_t s);
 void launch_upload_records(int slots, int n, const UploadSrc& src, const PArrays& P, int track_fp, void* rec,

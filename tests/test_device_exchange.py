@@ -116,3 +116,39 @@ def test_device_arrays_bad_mass_is_refused():
     torch.cuda.synchronize()
     st = s._lib.aep_set_particles(s._h, 300, *[_ptr(a) for a in bad[:8]], _ptr(bad[8], C.c_uint8))
     assert st == capi.AEP_INVALID_ARG
+
+
+@pytest.mark.parametrize("nside", [2, 9, 40])
+@pytest.mark.parametrize("want", [(0, 1, 2, 3, 4, 5, 6), (0, 3), (2, 6), (3, 4, 5), (6,), (0, 1, 2)])
+def test_mesh_state_on_the_device(nside, want):
+    """The mesh state from and into device arrays, whole records or single fields, is what the
+    host arrays give; fields that are not given keep their values."""
+    import torch
+
+    sc = scenes.cloth_drape(nside=nside, res=32)
+    s = HybridSolver(None, sc.grid, sc.params)
+    s.set_level_set(sc.levelset)
+    n = 33
+    _set(s, n, _state(n, False, 1))
+    s.set_lagrangian_mesh(sc.mesh)
+    s.step(1e-5)
+    nv, nf = len(sc.mesh.vertex_positions), len(sc.mesh.faces)
+    sizes = [3 * nv, 3 * nv, 9 * nv, 3 * nf, 3 * nf, 9 * nf, 9 * nf]
+
+    def get(make, which=range(7)):
+        out = [make(k) if f in which else None for f, k in enumerate(sizes)]
+        assert s._lib.aep_get_mesh(s._h, *[_ptr(a) for a in out]) == capi.AEP_OK
+        return out
+
+    before = get(np.empty)
+    on_dev = get(lambda k: torch.empty(k, dtype=torch.float64, device="cuda"), want)
+    for f in want:
+        np.testing.assert_array_equal(on_dev[f].cpu().numpy(), before[f])
+    rng = np.random.default_rng(5)
+    new = [(0.3 + 0.4 * rng.random(k)).astype(np.float32).astype(np.float64) for k in sizes]
+    dev = [torch.from_numpy(a).cuda() if f in want else None for f, a in enumerate(new)]
+    torch.cuda.synchronize()
+    assert s._lib.aep_set_mesh_state(s._h, nv, nf, *[_ptr(a) for a in dev]) == capi.AEP_OK
+    after = get(np.empty)
+    for f in range(7):
+        np.testing.assert_array_equal(after[f], new[f] if f in want else before[f])
