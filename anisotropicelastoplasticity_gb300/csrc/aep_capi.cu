@@ -85,7 +85,11 @@ struct aep_solver {
     GArrays G{};
     size_t nnodes = 0;
     int nblocks = 0;
+    // the counters of the current step and, zeroed, those of the next one: two in turn
     DevStats* dstats = nullptr;
+    DevStats* dstats_next = nullptr;
+    bool next_zeroed = false;
+    long long* dmovers = nullptr;  // of the last ordering, until the normalisation takes it
     double* staging = nullptr;
     size_t staging_bytes = 0;
     double* dforce = nullptr;  // dense f_i after a force-stage stop
@@ -465,7 +469,7 @@ cudaError_t order_particles(aep_solver* s) {
                 if (e != cudaSuccess) return e;
             }
             OrderBuffers b{s->keys, s->keys_sorted, s->perm, s->iota, s->mk, s->mj, s->mprev, s->mkeys, s->mslot, s->mpos,
-                           s->order_scratch, s->sort_tmp, s->sort_bytes, n, n / 4, s->key_bits, s->dstats};
+                           s->order_scratch, s->sort_tmp, s->sort_bytes, n, n / 4, s->key_bits, s->dmovers};
             cudaError_t e = order_graph_build(&s->order_graph, s->capture_stream, b);
             if (e != cudaSuccess) return e;
             s->order_graph_n = n;
@@ -474,7 +478,7 @@ cudaError_t order_particles(aep_solver* s) {
     }
     cudaError_t e = sort_pairs(s->sort_tmp, s->sort_bytes, s->keys, s->keys_sorted, s->iota, s->perm, n,
                                s->key_bits, s->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&s->dstats->movers, 0xFF, sizeof(long long), s->stream);  // -1
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->dmovers, 0xFF, sizeof(long long), s->stream);  // -1
     if (e == cudaSuccess) s->prev_sorted = true;
     return e;
 }
@@ -487,7 +491,10 @@ aep_status run_p2g(aep_solver* s) {
         s->dirty_grid = false;
     }
     const PArrays& P = s->P[s->cur];
-    CK(cudaMemsetAsync(s->dstats, 0, sizeof(DevStats), s->stream));
+    std::swap(s->dstats, s->dstats_next);
+    s->G.nactive = &s->dstats->nactive;
+    if (!s->next_zeroed) CK(cudaMemsetAsync(s->dstats, 0, sizeof(DevStats), s->stream));
+    s->next_zeroed = false;
     mark(s, AEP_PHASE_SORT);
     if (!s->keys_valid) {
         launch_keys(s->kp, P, (int)s->n, s->keys, s->dstats, s->stream);
@@ -512,8 +519,9 @@ aep_status run_p2g(aep_solver* s) {
     launch_p2g(s->kp, P, s->step_keys, s->step_perm, (int)s->n, s->G, s->slot_of, s->curidx_of, s->stream);
     CKLAUNCH();
     mark(s, AEP_PHASE_NORMALIZE);
-    launch_normalize(s->kp, s->G, s->dstats, s->grid_blocks, s->stream);
+    launch_normalize(s->kp, s->G, s->dstats, s->dstats_next, s->dmovers, s->grid_blocks, s->stream);
     CKLAUNCH();
+    s->next_zeroed = true;
     mark(s, AEP_PHASE_CLOTH_FORCE);
     return AEP_OK;
 }
@@ -589,6 +597,9 @@ aep_status aep_solver_create(const aep_grid_desc* grid, const aep_params* params
     CK(cudaMalloc(&s->G.flag, sizeof(uint32_t) * (size_t)s->nblocks));
     CK(cudaMalloc(&s->G.active, sizeof(int32_t) * (size_t)s->nblocks));
     CK(cudaMalloc(&s->dstats, sizeof(DevStats)));
+    CK(cudaMalloc(&s->dstats_next, sizeof(DevStats)));
+    CK(cudaMalloc(&s->dmovers, sizeof(long long)));
+    CK(cudaMemsetAsync(s->dmovers, 0, sizeof(long long), s->stream));
     s->G.nactive = &s->dstats->nactive;  // device address inside the counters
     CK(cudaMemsetAsync(s->G.acc, 0, sizeof(unsigned long long) * 4 * s->nnodes, s->stream));
     CK(cudaMemsetAsync(s->G.vel, 0, sizeof(float4) * s->nnodes, s->stream));
@@ -613,6 +624,8 @@ aep_status aep_solver_destroy(aep_solver* s) {
     cudaFree(s->G.flag);
     cudaFree(s->G.active);
     cudaFree(s->dstats);
+    cudaFree(s->dstats_next);
+    cudaFree(s->dmovers);
     cudaFree(s->dforce);
     cudaFree(s->harvest_count);
     cudaFree(s->queue_mem);

@@ -10,7 +10,8 @@ namespace aep {
 void launch_keys(const KParams& P, const PArrays& cur, int n, uint32_t* keys, DevStats* st, cudaStream_t s);
 void launch_p2g(const KParams& P, const PArrays& cur, const uint32_t* keys, const int32_t* perm, int n,
                 const GArrays& G, int32_t* slot_of, int32_t* curidx_of, cudaStream_t s);
-void launch_normalize(const KParams& P, const GArrays& G, DevStats* st, int grid_blocks, cudaStream_t s);
+void launch_normalize(const KParams& P, const GArrays& G, DevStats* st, DevStats* next, long long* movers,
+                      int grid_blocks, cudaStream_t s);
 void launch_cloth_force(const KParams& P, const PArrays& cur, const MeshArrays& M, float dt_force, cudaStream_t s);
 void launch_force(const KParams& P, const PArrays& cur, const uint32_t* keys, const int32_t* perm, int n,
                   const GArrays& G, float dt_force, DevStats* st, const MeshArrays& M, cudaStream_t s,
@@ -92,7 +93,7 @@ struct OrderBuffers {
     void* sort_tmp;
     size_t sort_bytes;
     int n, cap, key_bits;
-    DevStats* st;
+    long long* movers;  // out: their number, -1: full sort
 };
 size_t order_scratch_words(int n);
 cudaError_t order_graph_build(void** out, cudaStream_t capture_stream, const OrderBuffers& b);

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kFlagThreads, 2) k_flag_movers(const uint32_t*
                                                               uint32_t* __restrict__ mkeys, int32_t* __restrict__ mslot,
                                                               int32_t* __restrict__ mpos,
                                                               int32_t* __restrict__ counters,
-                                                              cudaGraphConditionalHandle h, DevStats* st) {
+                                                              cudaGraphConditionalHandle h, long long* movers) {
     __shared__ bool last;
     __shared__ int warp_sum[kFlagThreads / 32];
     const int j = blockIdx.x * kFlagThreads + threadIdx.x;
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kFlagThreads, 2) k_flag_movers(const uint32_t*
     }
     if (threadIdx.x == 0) {
         cudaGraphSetConditional(h, branch);
-        st->movers = branch == 2u ? -1ll : (long long)m;
+        *movers = branch == 2u ? -1ll : (long long)m;
         counters[0] = m;
         counters[1] = 0;
     }
@@ -503,7 +503,7 @@ cudaError_t order_graph_build(void** out, cudaStream_t cs, const OrderBuffers& b
     OG_CK(cudaStreamBeginCaptureToGraph(cs, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     OG_CK(cudaMemsetAsync(counters, 0, sizeof(int32_t), cs));
     k_flag_movers<<<nb, kFlagThreads, 0, cs>>>(b.keys, b.keys_sorted, n, b.cap, mask, blk, b.mk, b.mj, b.mprev, b.mkeys,
-                                               b.mslot, b.mpos, counters, h, b.st);
+                                               b.mslot, b.mpos, counters, h, b.movers);
     OG_CK(cudaGetLastError());
     cudaStreamCaptureStatus status;
     const cudaGraphNode_t* deps = nullptr;
