@@ -669,7 +669,7 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
     s->np = n;
     PArrays& P = s->P[s->cur];
     // Arrays in page-locked host or device memory are read by the conversion
-    // kernel directly; pageable ones are staged first (doubles): x 0, v 3n, B 6n,
+    // kernels directly; pageable ones are staged first (doubles): x 0, v 3n, B 6n,
     // Fe 15n, Fp 24n, m 33n, vol 34n, plastic 35n, material bytes at 36n.
     const size_t N = (size_t)n;
     cudaError_t e = cudaSuccess;
