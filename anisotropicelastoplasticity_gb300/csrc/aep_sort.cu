@@ -204,11 +204,18 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t* __res
     }
 }
 
+// the tile counts and totals ahead of the scratch pairs
+static size_t rs_hist_bytes(const RsPlan& p) {
+    return (sizeof(int32_t) * ((size_t)kRsBins * p.tiles + kRsBins) + 255) & ~(size_t)255;
+}
+
+// Scratch that serves every size up to n: a buffer is sized once for the largest.  The
+// tile counts of the longest sort of short tiles outweigh the pairs of a somewhat longer one.
 size_t sort_temp_bytes(int n, int key_bits) {
-    const RsPlan p = rs_plan(n, key_bits);
-    const size_t hist = sizeof(int32_t) * ((size_t)kRsBins * p.tiles + kRsBins);
-    const size_t pairs = (sizeof(uint32_t) + sizeof(int32_t)) * (size_t)std::max(n, 1);
-    return ((hist + 255) & ~(size_t)255) + pairs;
+    auto bytes = [&](int k) {
+        return rs_hist_bytes(rs_plan(k, key_bits)) + (sizeof(uint32_t) + sizeof(int32_t)) * (size_t)std::max(k, 1);
+    };
+    return n < kRsLarge ? bytes(n) : std::max(bytes(n), bytes(kRsLarge - 1));
 }
 
 cudaError_t sort_pairs(void* temp, size_t temp_bytes, const uint32_t* keys_in, uint32_t* keys_out,
@@ -218,8 +225,7 @@ cudaError_t sort_pairs(void* temp, size_t temp_bytes, const uint32_t* keys_in, u
     const RsPlan p = rs_plan(n, key_bits);
     int32_t* hist = static_cast<int32_t*>(temp);
     int32_t* totals = hist + (size_t)kRsBins * p.tiles;
-    const size_t hist_bytes = (sizeof(int32_t) * ((size_t)kRsBins * p.tiles + kRsBins) + 255) & ~(size_t)255;
-    uint32_t* tk = reinterpret_cast<uint32_t*>(static_cast<char*>(temp) + hist_bytes);
+    uint32_t* tk = reinterpret_cast<uint32_t*>(static_cast<char*>(temp) + rs_hist_bytes(p));
     int32_t* tv = reinterpret_cast<int32_t*>(tk + n);
     const uint32_t mask = (1u << p.radix) - 1u;
     const uint32_t* ik = keys_in;
