@@ -116,8 +116,9 @@ struct aep_solver {
     SolveState* solve = nullptr;
     // read back after every step of aep_solve, two steps in flight (pinned, [2])
     SolveState* solve_host = nullptr;
-    DevStats* stats_host = nullptr;
     cudaEvent_t solve_read[2] = {};
+    // written by the device within every step of aep_solve (pinned; k_solve_dt)
+    unsigned long long* solve_seen = nullptr;
     aep_solve_fn solve_fn = nullptr;
     void* solve_user = nullptr;
     int64_t max_steps = 0;
@@ -633,7 +634,7 @@ aep_status aep_solver_destroy(aep_solver* s) {
     cudaFreeHost(s->check_host);
     cudaFree(s->solve);
     cudaFreeHost(s->solve_host);
-    cudaFreeHost(s->stats_host);
+    cudaFreeHost(s->solve_seen);
     for (cudaEvent_t e : s->solve_read)
         if (e) cudaEventDestroy(e);
     for (int r = 0; r < aep_solver::kRing; ++r)
@@ -995,7 +996,7 @@ aep_status step_impl(aep_solver* s, double dt_force, double dt, int32_t stage, b
         return AEP_OK;
     }
     if (adaptive) {
-        launch_solve_dt(s->solve, 0, s->stream);
+        launch_solve_dt(s->solve, 0, s->dstats, s->solve_seen, s->stream);
         CKLAUNCH();
     }
     const float dtf = (float)dt_force;
@@ -1023,7 +1024,7 @@ aep_status step_impl(aep_solver* s, double dt_force, double dt, int32_t stage, b
         CKLAUNCH();
     }
     if (adaptive) {
-        launch_solve_dt(s->solve, 1, s->stream);
+        launch_solve_dt(s->solve, 1, s->dstats, s->solve_seen, s->stream);
         CKLAUNCH();
     }
     if (stage == AEP_STAGE_GRID) return AEP_OK;
@@ -1117,7 +1118,7 @@ aep_status aep_solve(aep_solver* s, double cfl, double maxt, double alpha) {
     if (!s->solve) {
         CK(cudaMalloc(&s->solve, sizeof(SolveState)));
         CK(cudaMallocHost(&s->solve_host, 2 * sizeof(SolveState)));
-        CK(cudaMallocHost(&s->stats_host, 2 * sizeof(DevStats)));
+        CK(cudaMallocHost(&s->solve_seen, sizeof(unsigned long long)));
         for (cudaEvent_t& e : s->solve_read) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     // the first P2G of solve computes densities and volumes (:853-855)
@@ -1129,35 +1130,41 @@ aep_status aep_solve(aep_solver* s, double cfl, double maxt, double alpha) {
     init.cfl = cfl;
     init.inv_hmin = 1.0 / hmin;
     CK(cudaMemcpyAsync(s->solve, &init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
+    *s->solve_seen = 0ull;  // the stream is idle since aep_init_volumes
     s->solve_last = aep_solve_state{};
     // A step's clock is read back while the next one already runs, where the next one is
-    // certain to follow: no callback may end the solve, and t, which only moves at the end
-    // of a frame, cannot move in the step in flight (Dt <= CFL / 300).  Waiting for every
-    // step before the launch of the next left the device idle between them (131,072
-    // particles, 24 steps and the exchange: 4.12 -> 3.86 ms).  Should the step in flight overflow, the
-    // one after it has run as well; the statistics kept are those of the overflow.
+    // certain to follow: no callback may end the solve, t, which only moves at the end of a
+    // frame, cannot move in the step in flight (Dt <= CFL / 300), and that step is past its
+    // normalisation without an overflow.  Waiting for the end of every step before the launch
+    // of the next left the device idle between them (snow: 77 -> 73 us a step at 512
+    // particles, 73 -> 70 at 32,768, 105 -> 98 at 131,072, 241 -> 237 at 524,288).
     double t = 0.0, inner = 0.0;  // after the last step read
     int64_t launched = 0, read = 0;
+    // whether step i (from 1) went through its normalisation without an overflow; waits until
+    // the device has said so, or until the step has ended, with or without an error
+    auto normalised = [&](int64_t i) {
+        const unsigned long long want = 2ull * (unsigned long long)i;
+        while (__atomic_load_n(s->solve_seen, __ATOMIC_ACQUIRE) < want &&
+               cudaEventQuery(s->solve_read[(i - 1) & 1]) == cudaErrorNotReady)
+            cudaGetLastError();  // not an error of the launches that follow
+        return __atomic_load_n(s->solve_seen, __ATOMIC_ACQUIRE) == want;
+    };
     for (;;) {
         aep_status launch = AEP_OK;
         while (launch == AEP_OK && launched - read < 2 && t <= maxt && (s->max_steps <= 0 || launched < s->max_steps) &&
-               (launched == read || (!s->solve_fn && inner + cfl / 3e2 < 1.0 / 60.0))) {
+               (launched == read || (!s->solve_fn && inner + cfl / 3e2 < 1.0 / 60.0 && normalised(launched)))) {
             launch = step_impl(s, 0.0, 0.0, AEP_STAGE_FULL, true);
             if (launch) break;
             const int k = (int)(launched++ & 1);
             CK(cudaMemcpyAsync(s->solve_host + k, s->solve, sizeof(SolveState), cudaMemcpyDeviceToHost, s->stream));
-            CK(cudaMemcpyAsync(s->stats_host + k, s->dstats, sizeof(DevStats), cudaMemcpyDeviceToHost, s->stream));
             CK(cudaEventRecord(s->solve_read[k], s->stream));
         }
         if (launched == read) return launch;
         const int k = (int)(read++ & 1);
         CK(cudaEventSynchronize(s->solve_read[k]));
-        if (s->stats_host[k].overflow) {
-            if (launched > read)
-                CK(cudaMemcpyAsync(s->dstats, s->stats_host + k, sizeof(DevStats), cudaMemcpyHostToDevice, s->stream));
-            CK(cudaStreamSynchronize(s->stream));
+        // no step follows an overflow: the word is still that step's
+        if (__atomic_load_n(s->solve_seen, __ATOMIC_ACQUIRE) == 2ull * (unsigned long long)read + 1ull)
             return fail(s, AEP_OVERFLOW, "fixed-point grid accumulator overflow");
-        }
         const SolveState& h = s->solve_host[k];
         t = h.t;
         inner = h.inner;

@@ -989,10 +989,15 @@ __global__ void k_query_weights(KParams P, PArrays cur, const int32_t* __restric
 // the force pass and grid update use the current Dt (:873, :877).  phase 1 (after
 // the grid update): Dt = CFL / max(300, max|v| / hmin) (:878) with the frame
 // clamp (:880-892); the G2P of this step and the force pass of the next use it.
+// Phase 0 also tells the host that step i (from 1) is past its normalisation, where the
+// accumulators are checked: 2 i, + 1 after an overflow, in a pinned word.  No step may follow
+// an overflow, and the step's end is too late to launch the next one.
 // Launched early, as its neighbours are: 4 us a step less than two plain launches.
-__global__ void k_solve_dt(SolveState* S, int phase) {
+__global__ void k_solve_dt(SolveState* S, int phase, const DevStats* st, unsigned long long* seen) {
     pdl_entry();
     if (phase == 0) {
+        *const_cast<volatile unsigned long long*>(seen) =
+            2ull * (unsigned long long)(S->steps + 1) + (st->overflow ? 1ull : 0ull);
         if (!S->initialized) {
             const double v = sqrt((double)__uint_as_float(S->vmax2[0]));
             S->Dt = S->cfl / fmax(3e2, v * S->inv_hmin);
@@ -2752,7 +2757,9 @@ void launch_fixed_vertices(const KParams& P, const PArrays& cur, const GArrays& 
     const long threads = (long)nfixed * 64 * 27;
     if (threads > 0) k_fixed_vertices<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(P, cur, G, M, fixed, nfixed);
 }
-void launch_solve_dt(SolveState* S, int phase, cudaStream_t s) { launch_pdl(k_solve_dt, 1, 1, 0, s, S, phase); }
+void launch_solve_dt(SolveState* S, int phase, const DevStats* st, unsigned long long* seen, cudaStream_t s) {
+    launch_pdl(k_solve_dt, 1, 1, 0, s, S, phase, st, seen);
+}
 void launch_query_weights(const KParams& P, const PArrays& cur, const int32_t* inv, const int64_t* ids, int count,
                           int64_t* nodes, double* w, double* g, cudaStream_t s) {
     const long threads = (long)count * 64;

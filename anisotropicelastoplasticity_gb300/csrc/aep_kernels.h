@@ -59,7 +59,7 @@ void launch_download_F_slots(int slots, int n, double* dst, float* const* F, con
 void launch_download_particles(int n, const DownloadDst& dst, const PArrays& P, const int32_t* inv, cudaStream_t s);
 void launch_fixed_vertices(const KParams& P, const PArrays& cur, const GArrays& G, const MeshArrays& M,
                            const int32_t* fixed, int nfixed, cudaStream_t s);
-void launch_solve_dt(SolveState* S, int phase, cudaStream_t s);
+void launch_solve_dt(SolveState* S, int phase, const DevStats* st, unsigned long long* seen, cudaStream_t s);
 void launch_query_weights(const KParams& P, const PArrays& cur, const int32_t* inv, const int64_t* ids, int count,
                           int64_t* nodes, double* w, double* g, cudaStream_t s);
 void launch_check_upload(int n, const double* m, const uint8_t* mat, unsigned long long* out, cudaStream_t s);

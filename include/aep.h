@@ -284,8 +284,9 @@ aep_status aep_set_max_steps(aep_solver* s, int64_t max_steps);
  * velocities before collision (:878, RegularGrid.cpp:188-200) and clamped to
  * end the 1/60 s frame (:880-892).  Dt and the frame clock live on the device;
  * the host reads them once per step, without a callback while the next step
- * already runs where that one is certain to follow (after AEP_OVERFLOW one step
- * more may have run).  alpha is accepted and unused, as in the reference (:739). */
+ * already runs where that one is certain to follow.  No step follows one that
+ * overflowed: the state after AEP_OVERFLOW is that step's.  alpha is accepted
+ * and unused, as in the reference (:739).                                      */
 aep_status aep_solve(aep_solver* s, double cfl, double maxt, double alpha);
 
 /* The state after the last step of the current or last aep_solve call. */
