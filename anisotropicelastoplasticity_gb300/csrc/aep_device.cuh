@@ -275,6 +275,9 @@ __device__ __forceinline__ void tile_origin(const KParams& P, uint32_t key, int 
 // (triggers at the start, and late: 65,536 vertices and 130,050 triangles 135.3 -> 125.4 us a
 // step, 200,000 particles 152.3 -> 145.5, 2,097,152 943 -> 929, 512 44.8 -> 43.8).  pdl_entry()
 // is for the small ones.  All are no-ops for a kernel launched without the attribute.
+// What such a kernel reads after its wait comes through plain pointers: the previous kernel
+// may write it while this one already runs, which const __restrict__ would deny (G2P's keys
+// in and out, besides, are one array in the steps without an ordering).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_entry() {
@@ -309,7 +312,7 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 // 16 threads each, then the rows y = 8.  A column's nodes along z lie 16 nodes apart inside
 // each of three node blocks, so a copy costs one instruction with a constant offset (with
 // a node index for each: force 1,314 -> 1,297 us, G2P 1,104 -> 1,099 at 8,388,608 particles).
-__device__ __forceinline__ void load_gather_tile(const KParams& P, const int org[3], const float4* __restrict__ src,
+__device__ __forceinline__ void load_gather_tile(const KParams& P, const int org[3], const float4* src,
                                                  float4* dst) {
     {
         const int x = threadIdx.x & 15, y = threadIdx.x >> 4;
@@ -341,7 +344,7 @@ __device__ __forceinline__ bool gather_offset(const int base[3], const int org[3
 }
 // flag t (t < 72) of the node blocks under the tile, two per block: 4 x 3 x 3 blocks from
 // one before org
-__device__ __forceinline__ bool tile_differs(const KParams& P, const int org[3], const uint8_t* __restrict__ flags, int t) {
+__device__ __forceinline__ bool tile_differs(const KParams& P, const int org[3], const uint8_t* flags, int t) {
     const int b = t >> 1, x = org[0] - 1 + (b & 3), y = org[1] - 1 + (b >> 2) % 3, z = org[2] - 1 + (b >> 2) / 3;
     if (x < 0 || y < 0 || z < 0 || x >= P.nb[0] || y >= P.nb[1] || z >= P.nb[2]) return false;
     return flags[2 * ((z * P.nb[1] + y) * P.nb[0] + x) + (t & 1)] != 0;
@@ -359,7 +362,7 @@ __device__ __forceinline__ bool stencil_differs(const int base[3], const int org
     return d;
 }
 // the same for any stencil, from the flags in global memory
-__device__ __forceinline__ bool grid_differs(const KParams& P, const int base[3], const uint8_t* __restrict__ flags) {
+__device__ __forceinline__ bool grid_differs(const KParams& P, const int base[3], const uint8_t* flags) {
     bool d = false;
     for (int z = base[2] >> 1; z <= (base[2] + 3) >> 1; ++z)
         for (int y = base[1] >> 2; y <= (base[1] + 3) >> 2; ++y)

@@ -116,10 +116,9 @@ __device__ __forceinline__ void mark_blocks(const KParams& P, const GArrays& G, 
 // bit from step to step.  T - S is far below 2^31 (FP32 weight-sum error and
 // roundings), so it is computed from the low 32 bits of T and of the node masses
 // with one 32-bit warp reduction.
-__global__ void __launch_bounds__(kP2GThreads, 6) k_p2g(KParams P, PArrays cur, const uint32_t* __restrict__ keys,
-                                                     const int32_t* __restrict__ perm, int n, int chunk, int share,
-                                                     GArrays G, int32_t* __restrict__ slot_of,
-                                                     int32_t* __restrict__ curidx_of) {
+__global__ void __launch_bounds__(kP2GThreads, 6) k_p2g(KParams P, PArrays cur, const uint32_t* keys,
+                                                        const int32_t* perm, int n, int chunk, int share, GArrays G,
+                                                        int32_t* slot_of, int32_t* curidx_of) {
     pdl_wait();
     __shared__ float4 sm4[(kP2GThreads / 32) * kP2GRegion];
     __shared__ unsigned long long tacc[4 * kP2GTileNodes];  // [channel][tile node]
@@ -507,7 +506,7 @@ __device__ __forceinline__ void gradient_tile(const float4* t, const float w[3][
     }
 }
 // the same sums in the same order from the grid (stencils outside the tile)
-__device__ __forceinline__ void gradient_grid(const KParams& P, const float4* __restrict__ f, const int base[3],
+__device__ __forceinline__ void gradient_grid(const KParams& P, const float4* f, const int base[3],
                                               const float w[3][4], const float dw[3][4], float Gm[9]) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) Gm[k] = 0.f;
@@ -572,7 +571,7 @@ __device__ void particle_stress_impulse(const KParams& P, const float Gm[9], con
 // stencil nodes with its own fixed-point atomics (integer sums: the order does
 // not matter).  Grid-stride over the list; usually empty.
 __global__ void k_force_fp64(KParams P, PArrays cur, GArrays G, float dt_force, DevStats* st,
-                             const int32_t* __restrict__ fp64_list, int fp64_cap) {
+                             const int32_t* fp64_list, int fp64_cap) {
     pdl_entry();
     dt_force = step_dt(P, dt_force, 0);
     const int count = min((int)st->force_fp64, fp64_cap);
@@ -589,7 +588,7 @@ __global__ void k_force_fp64(KParams P, PArrays cur, GArrays G, float dt_force, 
         for (int oz = 0; oz < 4; ++oz)
             for (int oy = 0; oy < 4; ++oy)
                 for (int ox = 0; ox < 4; ++ox) {
-                    const float4 v = __ldg(&G.vel[Y[oy] + Z[oz] + X[ox]]);
+                    const float4 v = G.vel[Y[oy] + Z[oz] + X[ox]];
                     const float g[3] = {dw[0][ox] * w[1][oy] * w[2][oz], w[0][ox] * dw[1][oy] * w[2][oz],
                                         w[0][ox] * w[1][oy] * dw[2][oz]};
                     const float vv[3] = {v.x, v.y, v.z};
@@ -635,9 +634,9 @@ __global__ void k_force_fp64(KParams P, PArrays cur, GArrays G, float dt_force, 
 }
 
 // impulse scatter: f_i -= sum_p stress_p grad w_ip (HS:356-366), stored as dt * f_i
-__global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur, const uint32_t* __restrict__ keys,
-                                                       const int32_t* __restrict__ perm, int n, GArrays G,
-                                                       float dt_force, DevStats* st, MeshArrays M,
+__global__ void __launch_bounds__(kFrcThreads, 6) k_force(KParams P, PArrays cur, const uint32_t* keys,
+                                                       const int32_t* perm, int n, GArrays G, float dt_force,
+                                                       DevStats* st, MeshArrays M,
                                                        int32_t* fp64_list, int fp64_cap, int share) {
     pdl_wait();
     // the grid tile, then (after a barrier) the warps' prep records in the same memory
@@ -1295,7 +1294,7 @@ __device__ __forceinline__ void gather_tile(const float4* t, const float w[3][4]
 }
 // The same sums in the same order from the grid (stencils outside the tile, cloth
 // elements); rows one after another, small code for a rare path
-__device__ __forceinline__ void gather_grid(const KParams& P, const float4* __restrict__ f, const int base[3],
+__device__ __forceinline__ void gather_grid(const KParams& P, const float4* f, const int base[3],
                                             const float w[3][4], const float dw[3][4], const float xi[3][4],
                                             Gathered& g) {
     float wxi[4];
@@ -1375,9 +1374,9 @@ constexpr int kG2PSmallPart = 64;  // particles per thread block of the small fo
 // half the particles.  Measured: 16.7 -> 13.4 us at 2,500 particles, 20.9 -> 18.7 at 16,000,
 // 18.2 -> 16.4 at 38,000; with twice the limit 22.0 -> 25.4 at 60,000.
 template <bool kDefer, bool kSmall>
-__global__ void __launch_bounds__(128, kSmall || !kDefer ? 4 : 5) k_g2p(KParams P, PArrays cur, PArrays nxt, const int32_t* __restrict__ perm,
-                                             int n, GArrays G, float dt, uint32_t* __restrict__ keys_next,
-                                             DevStats* st, Harvest H, const uint32_t* __restrict__ keys_sorted,
+__global__ void __launch_bounds__(128, kSmall || !kDefer ? 4 : 5) k_g2p(KParams P, PArrays cur, PArrays nxt, const int32_t* perm,
+                                             int n, GArrays G, float dt, uint32_t* keys_next, DevStats* st,
+                                             Harvest H, const uint32_t* keys_sorted,
                                              MlpQueue Qu) {
     pdl_wait();
     constexpr int kPart = kSmall ? kG2PSmallPart : 128;  // particles of the block
@@ -1877,7 +1876,7 @@ __global__ void __launch_bounds__(kFinThreads) k_mlp_finish(KParams P, PArrays c
 // elements record [r13, r23, r33 - 1, cap ratio, 2, projected - trial (3)].
 template <bool kMlp>
 __global__ void __launch_bounds__(128) k_cloth_g2p(KParams P, PArrays nxt, MeshArrays M,
-                                                   uint32_t* __restrict__ keys_next, DevStats* st, Harvest H,
+                                                   uint32_t* keys_next, DevStats* st, Harvest H,
                                                    MlpParams mlp, float tol_rel, float tol_abs) {
     pdl_entry();
     extern __shared__ __align__(16) unsigned char smem_raw[];

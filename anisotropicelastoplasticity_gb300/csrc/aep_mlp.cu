@@ -106,12 +106,10 @@ __device__ __forceinline__ float dsilu(float z) {
 // gradients, serial sums over 64 rows, are left for the end, each layer on its own warps.
 // Measured (16,384 rows, one Adam step with its reduction): 95 -> 20 us against single
 // 2-byte fragment loads from unpadded rows.
-__global__ void __launch_bounds__(kTrainThreads, 2) k_mlp_train_tile(const float* __restrict__ params,
-                                                                     const bf16* __restrict__ wb,
+__global__ void __launch_bounds__(kTrainThreads, 2) k_mlp_train_tile(const float* params, const bf16* wb,
                                                                      const float* __restrict__ rec, int n, int row0,
-                                                                     int row_end, int rows_total,
-                                                                     float* __restrict__ part,
-                                                                     float* __restrict__ part_loss) {
+                                                                     int row_end, int rows_total, float* part,
+                                                                     float* part_loss) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
@@ -317,10 +315,9 @@ struct AdamArgs {
 constexpr int kReduceParams = 32;
 constexpr int kReduceSplit = 8;
 template <bool kAdam>
-__global__ void __launch_bounds__(kReduceParams * kReduceSplit) k_mlp_reduce(const float* __restrict__ part,
-                                                                            const float* __restrict__ part_loss,
-                                                                            int blocks, float* __restrict__ grad,
-                                                                            float* __restrict__ loss, int accumulate,
+__global__ void __launch_bounds__(kReduceParams * kReduceSplit) k_mlp_reduce(const float* part,
+                                                                            const float* part_loss, int blocks,
+                                                                            float* grad, float* loss, int accumulate,
                                                                             AdamArgs A) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float ps[kReduceSplit][kReduceParams + 1];
