@@ -410,26 +410,40 @@ aep_status download(aep_solver* s, double* dst, int count, int mode, float* cons
     return AEP_OK;
 }
 
-// Readback into device memory goes by way of records from this many values per item: a
-// record costs 27 x 4 + 2 x 128 bytes whatever is asked for, a value read on its own a
-// 32-byte sector.
-constexpr int kRecordValues = 12;
+// Which exchanges with device memory go by way of records.  A record costs 27 x 4 + 2 x 128
+// bytes whatever is asked for and one kernel more; a value read on its own costs a 32-byte
+// sector.  Measured, us of a call by records / in the caller's order:
+//   readback of 26 values: 23.5 / 21.7 for 8,192 items, 24.5 / 24.8 for 32,768, 26.5 / 28.7
+//     for 65,536, 126 / 165 for 1,000,000; with F_P (35 values), a kernel more: 30.8 / 26.9
+//     for 32,768, 38 / 38 for 100,003, 59 / 70 for 262,144
+//   readback of 12 values: 19 / 17 for 8,192, 100 / 85 for 1,000,000; of 15: 106 / 103; of
+//     18: 21.9 / 22.8 for 65,536, 114 / 120 for 1,000,000
+//   upload: 34 / 27 for 2,000, 34.6 / 34.6 for 32,768, 34.4 / 38.0 for 65,536, 134 / 208 for
+//     1,000,000; with F_P: 38 / 36 for 32,768, 40 / 47 for 65,536
+constexpr int kRecordValues = 16;
+constexpr int64_t kRecordReadback = 32768, kRecordReadbackFp = 100000, kRecordUpload = 40000;
 
-// whether mesh state goes by way of records: every array given is device memory, and a
-// vertex or an element has that many values
+// Mesh state by way of records: two kernels over every item, against one for each array given
+// (and one for the inverse of the ids).  All seven arrays: 24 / 46 us for 4,225 vertices (their
+// triangles are twice as many), 37 / 58 for 66,049, 98 / 119 for 263,169, 332 / 337 for
+// 1,050,625; three of the vertices': 22 / 26 for 16,641, 31 / 28 for 66,049, 78 / 39 for
+// 263,169; five of both: 23 / 27, 32 / 33 and 88 / 75.
+constexpr int kRecordMeshArrays = 3, kRecordMeshArraysLarge = 6;
+constexpr int64_t kRecordMeshLarge = 150000;  // items
+
+// whether mesh state goes by way of records (every array given has to be device memory)
 template <typename T>
 bool mesh_by_records(const MeshFields<T>& m) {
-    const T* const all[7] = {m.xv, m.vv, m.Bv, m.xe, m.ve, m.Be, m.d};
-    const int cnt[7] = {3, 3, 9, 3, 3, 9, 9};
-    int values[2] = {0, 0};
-    for (int f = 0; f < 7; ++f)
-        if (all[f]) {
-            bool on_device = false;
-            device_alias(all[f], &on_device);
-            if (!on_device) return false;
-            values[f >= 3] += cnt[f];
-        }
-    return std::max(values[0], values[1]) >= kRecordValues;
+    T* const all[] = {m.xv, m.vv, m.Bv, m.xe, m.ve, m.Be, m.d};
+    int arrays = 0;
+    for (T* a : all) {
+        if (!a) continue;
+        bool on_device = false;
+        device_alias(a, &on_device);
+        if (!on_device) return false;
+        ++arrays;
+    }
+    return arrays >= ((int64_t)m.nv + m.nf < kRecordMeshLarge ? kRecordMeshArrays : kRecordMeshArraysLarge);
 }
 
 aep_status check_overflow(aep_solver* s) {
@@ -695,7 +709,7 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
     // the whole upload and its validation (bad masses, unknown tags, largest mass)
     // in one launch, read back with the final synchronisation
     CK(cudaMemsetAsync(s->check, 0, 2 * sizeof(unsigned long long), s->stream));
-    if (keep_order && all_on_device) {
+    if (keep_order && all_on_device && n >= kRecordUpload) {
         // by way of records, in the staging buffer (16 of its 37 doubles per item; unused here)
         launch_upload_records((int)s->n, (int)n, src, P, s->prm.track_plastic_F, s->staging, s->check, s->stream);
     } else {
@@ -1493,7 +1507,7 @@ aep_status aep_get_particles(aep_solver* s, int64_t n, double* x, double* v, dou
             values += f == 4 ? 0 : (int)cnt[f];
         }
     const DownloadDst dst{dev[0], dev[1], dev[2], dev[3], dev[4], dev[5], dev[6]};
-    if (all_on_device && values >= kRecordValues) {
+    if (all_on_device && values >= kRecordValues && np >= (Fp ? kRecordReadbackFp : kRecordReadback)) {
         launch_download_records((int)s->n, (int)np, dst, P, s->staging, s->stream);
         CKLAUNCH();
     } else {

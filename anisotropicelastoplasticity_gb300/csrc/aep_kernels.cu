@@ -2023,48 +2023,59 @@ __global__ void k_volumes(KParams P, PArrays cur, const int32_t* __restrict__ pe
 // ===================================================================================
 // layout conversion: reference FP64 layouts <-> device FP32 structure of arrays.
 // The device's item order is random against the caller's, so one side of every copy is random:
-//   host memory (k_upload_particles, k_download_particles, k_upload, k_download): one thread
-//     per item and group of fields (blockIdx.y: the group, the slow index, so one group's
-//     arrays fill the L2 while it runs), in the caller's order, so page-locked host memory
-//     streams over the host link at full width; the 3x3 matrices, 72 bytes per item, pass
-//     through shared memory for the same reason.
+//   k_upload_particles, k_download_particles, k_upload, k_download: in the caller's order, one
+//     thread per value (the uploads of particles: four values of a column, and matrices 128
+//     items at a time through shared memory), field after field: page-locked host memory
+//     streams over the host link at full width, and a field's device arrays stay in the L2
+//     while it is moved.  Measured against a thread per item and three fields: readback of
+//     x and v of 4,000,000 items 175 -> 161 us, of all fields of 2,000 23.3 -> 21.2 (by
+//     records); upload of 4,000,000 393 -> 294.
 //   device memory (k_pack_items + k_items_to_slots, k_slots_to_items + k_unpack_items): by
 //     way of 128-byte FP32 records, one per item in the caller's order.  The caller's arrays
 //     and the device's are then both read and written in order, and the random side moves
 //     whole records, four full sectors each; single values would cost a 32-byte sector each
 //     (15 of the 27 values of an item are columns of N x 3 arrays), and the L2 takes only 27
-//     to 50 partial sectors per clock (measured).
-// Measured, 7,604,222 particles + 784,386 cloth items on device arrays: upload 3.7 ms for one kernel
-// in the caller's order, 2.05 for one in slot order, 1.08 for records; readback (with the
-// caller's own FP64 -> FP32 pass) 2.8, 2.4 and 1.7 ms; 2,097,152 particles: upload and readback
-// 0.96 ms in slot order, 0.73 for records; 262,144: 0.24 for both
+//     to 50 partial sectors per clock (measured).  7,604,222 particles + 784,386 cloth items:
+//     upload 3.7 -> 1.08 ms, readback (with the caller's own FP64 -> FP32 pass) 2.8 -> 1.7.
+//     The callers choose: few items or fields are faster in the caller's order.
 constexpr int kConvThreads = 256;
-// fields per group of the readback in the caller's order: as many as the L2 holds
-constexpr long kConvL2Bytes = 48l << 20;
+
+// the arrays of one field set: component c at f + c * stride
+struct FieldSet {
+    float* f;
+    long stride;
+};
+// Value c of item q in the b-th block of up to 9 columns of n values, nb blocks (conv_blocks)
+// each; false outside the column.  A warp's 32 values begin at a multiple of 128 bytes from
+// the first column's start, whatever n is: over the host link a partial line costs a whole one
+// (15 values of 263,169 vertices into page-locked memory 228 -> 192 us).
+constexpr int kConvAlign = 16;
+__device__ __forceinline__ int conv_shift(int c, long n) { return (int)(c * n & (kConvAlign - 1)); }
+__device__ __forceinline__ bool conv_column(int b, int nb, int n, int& q, int& c) {
+    c = b / nb;
+    q = (b - c * nb) * kConvThreads + threadIdx.x - conv_shift(c, n);
+    return q >= 0 && q < n;
+}
+static int conv_blocks(int n, int per) { return (int)(((long)n + kConvAlign - 1 + per - 1) / per); }
+// the same of n items of 9 values each
+__device__ __forceinline__ bool conv_matrix(int b, int n, int& q, int& c) {
+    const unsigned i = (unsigned)(b % 9) * kConvThreads + threadIdx.x;
+    q = b / 9 * kConvThreads + (int)(i / 9u);
+    c = (int)(i % 9u);
+    return q < n;
+}
+__device__ __forceinline__ int transposed(int c) { return 3 * (c % 3) + c / 3; }
 
 // host-layout doubles -> FP32, one field set; item q goes to slot map[q] (or q).
-// mode 0: N x 3 column-major (1 group); 1: affine momenta, 3 blocks of N x 3, block a =
-// row a; 2: 3x3 column-major per item; 3: scalar; 4: element directions, 3 blocks of
-// N x 3, block c = column c (1, 2, 4: 3 groups)
-struct FieldPtrs {
-    float* f[9];
-};
-__device__ __forceinline__ long conv_index(int mode, long n, int g, int i, long q) {
-    return mode == 2 ? 9 * q + 3 * g + i : (3 * g + i) * n + q;
-}
-__device__ __forceinline__ int conv_field(int mode, int g, int i) { return mode == 2 || mode == 4 ? 3 * i + g : 3 * g + i; }
-
-__global__ void __launch_bounds__(kConvThreads) k_upload(int n, int mode, const double* __restrict__ src, FieldPtrs d,
-                                                         const int32_t* __restrict__ map) {
-    const int q = blockIdx.x * kConvThreads + threadIdx.x, g = blockIdx.y;
-    if (q >= n) return;
+// mode 0: N x 3 column-major; 1: affine momenta, 3 blocks of N x 3, block a = row a;
+// 2: 3x3 column-major per item; 3: scalar; 4: element directions, 3 blocks of N x 3,
+// block c = column c
+__global__ void __launch_bounds__(kConvThreads) k_upload(int n, int nb, int mode, const double* __restrict__ src,
+                                                         FieldSet d, const int32_t* __restrict__ map) {
+    int q, c;
+    if (!(mode == 2 ? conv_matrix(blockIdx.x, n, q, c) : conv_column(blockIdx.x, nb, n, q, c))) return;
     const int p = map ? map[q] : q;
-    if (mode == 3) {
-        d.f[0][p] = (float)src[q];
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) d.f[conv_field(mode, g, i)][p] = (float)src[conv_index(mode, n, g, i, q)];
+    d.f[(mode == 2 || mode == 4 ? transposed(c) : c) * d.stride + p] = (float)src[mode == 2 ? 9l * q + c : (long)c * n + q];
 }
 
 // m, vol, plastic (snow: J_P) and material of one item, FP32; the checks' inputs are returned
@@ -2114,39 +2125,64 @@ __device__ __forceinline__ void upload_check(unsigned long long mx, unsigned lon
     }
 }
 
-// The particle uploads of aep_set_particles in one launch, in the caller's order: groups
-// 0 x, 1 v, 2-4 B (row), 5 the item fields, 6 Fe, 7 F_P (launched with track_plastic_F and
-// a given F_P)
-__global__ void __launch_bounds__(kConvThreads) k_upload_particles(int n, UploadSrc src, PArrays P,
+// The particle uploads of aep_set_particles in one launch, in the caller's order: the item
+// fields, x, v and B (nb blocks per column), Fe, F_P (with track_plastic_F and a given F_P;
+// kConvItems items per block, through shared memory: their components go to nine arrays)
+constexpr int kConvItems = 128, kConvPer = 4;
+__global__ void __launch_bounds__(kConvThreads) k_upload_particles(int n, int nb, int nc, UploadSrc src, PArrays P,
                                                                    const int32_t* __restrict__ map, int track_fp,
                                                                    unsigned long long* check) {
-    __shared__ double sm[9 * kConvThreads];
-    const int q0 = blockIdx.x * kConvThreads, q = q0 + threadIdx.x, g = blockIdx.y;
-    const bool live = q < n;
+    __shared__ float sm[9 * kConvItems];
+    int b = blockIdx.x, q, c;
     const long N = n;
-    const int p = live ? (map ? map[q] : q) : 0;
-    if (g == 5) {  // block-uniform
+    if (b < nb) {
         unsigned long long mx = 0ull, bad = 0ull;
-        if (live) {
+        if (conv_column(b, nb, n, q, c)) {
+            const int p = map ? map[q] : q;
             P.id[p] = q;
             store_item(P, p, item_fields(src, q, track_fp, mx, bad), track_fp && !src.Fp);
         }
         upload_check(mx, bad, check);
-    } else if (g > 5) {
-        const double* f = (g == 6 ? src.Fe : src.Fp) + 9l * q0;
-        const int words = 9 * min(kConvThreads, n - q0);
-        for (int i = threadIdx.x; i < words; i += kConvThreads) sm[i] = f[i];
-        __syncthreads();
-        if (live)
+        return;
+    }
+    b -= nb;
+    if (b < 15 * nc) {
+        c = b / nc;
+        const int a = c < 3 ? c : c < 6 ? c - 3 : c - 6;
+        const double* const f = c < 3 ? src.x : c < 6 ? src.v : src.B;
+        float* const d = c < 3 ? P.x[a] : c < 6 ? P.v[a] : P.B[a];
+        q = (b - c * nc) * kConvThreads * kConvPer + threadIdx.x - conv_shift(a, n);
+        float val[kConvPer];
 #pragma unroll
-            for (int c = 0; c < 9; ++c) (g == 6 ? P.F : P.Fp)[3 * (c % 3) + c / 3][p] = (float)sm[9 * threadIdx.x + c];
-    } else if (live) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            if (g == 0) P.x[i][p] = (float)src.x[i * N + q];
-            else if (g == 1) P.v[i][p] = src.v ? (float)src.v[i * N + q] : 0.0f;
-            else P.B[3 * (g - 2) + i][p] = src.B ? (float)src.B[(3 * (g - 2) + i) * N + q] : 0.0f;
+        for (int k = 0; k < kConvPer; ++k) {
+            const int i = q + k * kConvThreads;
+            val[k] = f && i >= 0 && i < n ? (float)f[a * N + i] : 0.0f;
         }
+#pragma unroll
+        for (int k = 0; k < kConvPer; ++k) {
+            const int i = q + k * kConvThreads;
+            if (i >= 0 && i < n) d[map ? map[i] : i] = val[k];
+        }
+        return;
+    }
+    b -= 15 * nc;
+    const int nm = (n + kConvItems - 1) / kConvItems;
+    const bool fe = b < nm;
+    const int q0 = (fe ? b : b - nm) * kConvItems, items = min(kConvItems, n - q0);
+    const double* f = (fe ? src.Fe : src.Fp) + 9l * q0;
+    float* const d = fe ? P.F[0] : P.Fp[0];
+    const long stride = P.F[1] - P.F[0];
+#pragma unroll
+    for (int k = 0; k < 9 * kConvItems; k += kConvThreads) {
+        const int i = k + threadIdx.x;
+        if (i < 9 * items) sm[i] = (float)f[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 9 * kConvItems; k += kConvThreads) {
+        const int i = k + threadIdx.x, t = i % kConvItems;
+        c = i / kConvItems;
+        if (c < 9 && t < items) d[transposed(c) * stride + (map ? map[q0 + t] : q0 + t)] = sm[9 * t + c];
     }
 }
 
@@ -2249,12 +2285,12 @@ __global__ void __launch_bounds__(kRecThreads) k_items_to_slots(int slots, int n
 
 // F_P from a device array into the slots: 72 bytes per item
 __global__ void __launch_bounds__(kConvThreads) k_upload_F_slots(int slots, int n, const double* __restrict__ src,
-                                                                 FieldPtrs F, const int32_t* __restrict__ id) {
+                                                                 FieldSet F, const int32_t* __restrict__ id) {
     const int p = blockIdx.x * kConvThreads + threadIdx.x;
     const int q = p < slots ? id[p] : n;
     if (q >= n) return;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) F.f[3 * (c % 3) + c / 3][p] = (float)src[9l * q + c];
+    for (int c = 0; c < 9; ++c) F.f[transposed(c) * F.stride + p] = (float)src[9l * q + c];
 }
 
 // the slots' state of the ids [id0, id0 + n) into records
@@ -2318,45 +2354,36 @@ __global__ void __launch_bounds__(kRecThreads) k_unpack_items(int n, float4* __r
         if (32 * k + lane < words) dst.Fe[9l * q0 + 32 * k + lane] = (double)f[32 * k + lane];
 }
 
-// The particle readback of aep_get_particles, in the caller's order: one thread per item
-// and group, the groups of the requested fields (four bits each, blockIdx.y picks one):
-// 0 x, 1 v, 2-4 B (row), 5 the volume and the plastic scalar, 6 Fe, 7 F_P; inv[id] = slot.
-// split: x, v and B one field at a time (blockIdx.z)
-__global__ void __launch_bounds__(kConvThreads) k_download_particles(int n, unsigned groups, int split, DownloadDst dst,
-                                                                     PArrays P, const int32_t* __restrict__ inv) {
-    __shared__ double sm[9 * kConvThreads];
-    const int y = split ? blockIdx.y / 3 : blockIdx.y, z = split ? blockIdx.y % 3 : 0;
-    const int q0 = blockIdx.x * kConvThreads, q = q0 + threadIdx.x, g = (int)(groups >> (4 * y)) & 15;
-    const bool live = q < n;
-    const long N = n;
-    const int p = live ? inv[q] : 0;
-    if (g >= 5 && z > 0) return;  // block-uniform: these groups are not split
-    if (g > 5) {
-#pragma unroll
-        for (int c = 0; c < 9; ++c)
-            if (live) sm[9 * threadIdx.x + c] = (double)(g == 6 ? P.F : P.Fp)[3 * (c % 3) + c / 3][p];
-        __syncthreads();
-        double* f = (g == 6 ? dst.Fe : dst.Fp) + 9l * q0;
-        const int words = 9 * min(kConvThreads, n - q0);
-        for (int i = threadIdx.x; i < words; i += kConvThreads) f[i] = sm[i];
-    } else if (!live) {
-    } else if (g == 5) {
-        if (dst.vol) dst.vol[q] = (double)P.vol[p];
-        if (dst.plastic) dst.plastic[q] = (double)P.plastic[p];
-    } else {
-        const int first = split ? z : 0, last = split ? z + 1 : 3;
-        for (int i = first; i < last; ++i) {
-            const float* f = g == 0 ? P.x[i] : g == 1 ? P.v[i] : P.B[3 * (g - 2) + i];
-            double* d = g == 0 ? dst.x : g == 1 ? dst.v : dst.B + 3 * (g - 2) * N;
-            d[i * N + q] = (double)f[p];
+// The particle readback of aep_get_particles in one launch, in the caller's order: the columns
+// of the requested x, v, B, volume and plastic scalar (nb blocks each), then Fe and F_P;
+// inv[id] = slot
+__global__ void __launch_bounds__(kConvThreads) k_download_particles(int n, int nb, DownloadDst dst, PArrays P,
+                                                                     const int32_t* __restrict__ inv) {
+    int b = blockIdx.x, q, c;
+    const long stride = P.F[1] - P.F[0];
+    // whether the block is one of the k columns (or the matrices, k = 0) of a requested field
+    auto field = [&](double* d, const float* s, int k) {
+        const int blocks = (k ? k : 9) * nb;
+        if (!d) return false;
+        if (b >= blocks) {
+            b -= blocks;
+            return false;
         }
-    }
+        if (k) {
+            if (conv_column(b, nb, n, q, c)) d[(long)c * n + q] = (double)s[c * stride + inv[q]];
+        } else {
+            if (conv_matrix(b, n, q, c)) d[9l * q + c] = (double)s[transposed(c) * stride + inv[q]];
+        }
+        return true;
+    };
+    field(dst.x, P.x[0], 3) || field(dst.v, P.v[0], 3) || field(dst.B, P.B[0], 9) || field(dst.Fe, P.F[0], 0) ||
+        field(dst.Fp, P.Fp[0], 0) || field(dst.vol, P.vol, 1) || field(dst.plastic, P.plastic, 1);
 }
 
 // F_E (or F_P) into a device array from the slots' order: a warp's 32 matrices go through
 // shared memory and leave as 72-byte pieces, nine lanes each
 __global__ void __launch_bounds__(kConvThreads) k_download_F_slots(int slots, int n, double* __restrict__ dst,
-                                                                   FieldPtrs F, const int32_t* __restrict__ id) {
+                                                                   FieldSet F, const int32_t* __restrict__ id) {
     __shared__ double sm[9 * kConvThreads];
     __shared__ int32_t sq[kConvThreads];
     const int p = blockIdx.x * kConvThreads + threadIdx.x, w0 = threadIdx.x & ~31, lane = threadIdx.x & 31;
@@ -2364,7 +2391,7 @@ __global__ void __launch_bounds__(kConvThreads) k_download_F_slots(int slots, in
     sq[threadIdx.x] = q;
     if (q < n)
 #pragma unroll
-        for (int c = 0; c < 9; ++c) sm[9 * threadIdx.x + c] = (double)F.f[3 * (c % 3) + c / 3][p];
+        for (int c = 0; c < 9; ++c) sm[9 * threadIdx.x + c] = (double)F.f[transposed(c) * F.stride + p];
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
@@ -2455,19 +2482,15 @@ __global__ void __launch_bounds__(kRecThreads) k_unpack_mesh(MeshFields<double> 
     }
 }
 
-// FP32 -> host-layout doubles for ids [id_lo, id_lo + count), one field set (modes as in
+// FP32 -> host-layout doubles for ids [id_lo, id_lo + n), one field set (modes as in
 // k_upload); inv[id] = slot
-__global__ void __launch_bounds__(kConvThreads) k_download(int count, int mode, const int32_t* __restrict__ inv,
-                                                           int id_lo, double* __restrict__ dst, FieldPtrs s) {
-    const int q = blockIdx.x * kConvThreads + threadIdx.x, g = blockIdx.y;
-    if (q >= count) return;
+__global__ void __launch_bounds__(kConvThreads) k_download(int n, int nb, int mode, const int32_t* __restrict__ inv,
+                                                           int id_lo, double* __restrict__ dst, FieldSet s) {
+    int q, c;
+    if (!(mode == 2 ? conv_matrix(blockIdx.x, n, q, c) : conv_column(blockIdx.x, nb, n, q, c))) return;
     const int p = inv[id_lo + q];
-    if (mode == 3) {
-        dst[q] = (double)s.f[0][p];
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) dst[conv_index(mode, count, g, i, q)] = (double)s.f[conv_field(mode, g, i)][p];
+    dst[mode == 2 ? 9l * q + c : (long)c * n + q] =
+        (double)s.f[(mode == 2 || mode == 4 ? transposed(c) : c) * s.stride + p];
 }
 
 __global__ void k_init_particles(int n, PArrays cur, const uint8_t* __restrict__ mat_in, int has_fp, int track_fp,
@@ -2684,23 +2707,20 @@ void launch_volumes(const KParams& P, const PArrays& cur, const int32_t* perm, i
                     cudaStream_t s) {
     if (n > 0) k_volumes<<<blocks_for(n, 128), 128, 0, s>>>(P, cur, perm, n, G);
 }
-static FieldPtrs field_ptrs(float* const* f, int mode) {
-    FieldPtrs r{};
-    for (int k = 0; k < (mode == 3 ? 1 : mode == 0 ? 3 : 9); ++k) r.f[k] = f[k];
-    return r;
-}
-static dim3 conv_grid(int n, int groups) { return dim3((unsigned)blocks_for(n, kConvThreads), (unsigned)groups); }
-static int conv_groups(int mode) { return mode == 0 || mode == 3 ? 1 : 3; }
+static FieldSet field_set(float* const* f, int mode) { return {f[0], mode == 3 ? 0l : (long)(f[1] - f[0])}; }
+static int conv_columns(int mode) { return mode == 3 ? 1 : mode == 0 ? 3 : 9; }
 
 void launch_upload(int n, int mode, const double* src, float* const* dst, cudaStream_t s, const int32_t* map) {
+    const int nb = conv_blocks(n, kConvThreads);
     if (n > 0)
-        k_upload<<<conv_grid(n, conv_groups(mode)), kConvThreads, 0, s>>>(n, mode, src, field_ptrs(dst, mode), map);
+        k_upload<<<conv_columns(mode) * nb, kConvThreads, 0, s>>>(n, nb, mode, src, field_set(dst, mode), map);
 }
 void launch_upload_particles(int n, const UploadSrc& src, const PArrays& P, const int32_t* map, int track_fp,
                              unsigned long long* check, cudaStream_t s) {
+    const int nb = conv_blocks(n, kConvThreads), nc = conv_blocks(n, kConvThreads * kConvPer);
     if (n > 0)
-        k_upload_particles<<<conv_grid(n, (track_fp && src.Fp) ? 8 : 7), kConvThreads, 0, s>>>(n, src, P, map,
-                                                                                               track_fp, check);
+        k_upload_particles<<<nb + 15 * nc + ((track_fp && src.Fp) ? 2 : 1) * blocks_for(n, kConvItems), kConvThreads, 0,
+                             s>>>(n, nb, nc, src, P, map, track_fp, check);
 }
 void launch_upload_records(int slots, int n, const UploadSrc& src, const PArrays& P, int track_fp, void* rec,
                            unsigned long long* check, cudaStream_t s) {
@@ -2709,7 +2729,7 @@ void launch_upload_records(int slots, int n, const UploadSrc& src, const PArrays
     k_pack_items<<<blocks_for(n, kRecThreads), kRecThreads, 0, s>>>(n, src, r, track_fp, check);
     k_items_to_slots<<<blocks_for(slots, kRecThreads), kRecThreads, 0, s>>>(slots, n, r, P, track_fp && !src.Fp);
     if (track_fp && src.Fp)
-        k_upload_F_slots<<<blocks_for(slots, kConvThreads), kConvThreads, 0, s>>>(slots, n, src.Fp, field_ptrs(P.Fp, 2),
+        k_upload_F_slots<<<blocks_for(slots, kConvThreads), kConvThreads, 0, s>>>(slots, n, src.Fp, field_set(P.Fp, 2),
                                                                                   P.id);
 }
 void launch_download_records(int slots, int n, const DownloadDst& dst, const PArrays& P, void* rec, cudaStream_t s) {
@@ -2731,25 +2751,14 @@ void launch_download_mesh(int slots, int id0, const MeshFields<double>& m, const
     k_unpack_mesh<<<blocks_for(m.nv + m.nf, kRecThreads), kRecThreads, 0, s>>>(m, r);
 }
 void launch_download_particles(int n, const DownloadDst& dst, const PArrays& P, const int32_t* inv, cudaStream_t s) {
-    unsigned groups = 0;
-    int count = 0;
-    auto add = [&](bool want, int first, int k) {
-        for (int g = first; want && g < first + k; ++g) groups |= (unsigned)g << (4 * count++);
-    };
-    add(dst.x, 0, 1);
-    add(dst.v, 1, 1);
-    add(dst.B, 2, 3);
-    add(dst.vol || dst.plastic, 5, 1);
-    add(dst.Fe, 6, 1);
-    add(dst.Fp, 7, 1);
-    const int split = 12l * n <= kConvL2Bytes ? 0 : 1;  // three 4-byte fields
-    if (n > 0 && count > 0)
-        k_download_particles<<<conv_grid(n, split ? 3 * count : count), kConvThreads, 0, s>>>(n, groups, split, dst, P,
-                                                                                              inv);
+    const int nb = conv_blocks(n, kConvThreads);
+    const int columns = (dst.x ? 3 : 0) + (dst.v ? 3 : 0) + (dst.B ? 9 : 0) + (dst.vol ? 1 : 0) + (dst.plastic ? 1 : 0) +
+                        (dst.Fe ? 9 : 0) + (dst.Fp ? 9 : 0);
+    if (n > 0 && columns > 0) k_download_particles<<<columns * nb, kConvThreads, 0, s>>>(n, nb, dst, P, inv);
 }
 void launch_download_F_slots(int slots, int n, double* dst, float* const* F, const int32_t* id, cudaStream_t s) {
     if (slots > 0)
-        k_download_F_slots<<<blocks_for(slots, kConvThreads), kConvThreads, 0, s>>>(slots, n, dst, field_ptrs(F, 2), id);
+        k_download_F_slots<<<blocks_for(slots, kConvThreads), kConvThreads, 0, s>>>(slots, n, dst, field_set(F, 2), id);
 }
 void launch_fixed_vertices(const KParams& P, const PArrays& cur, const GArrays& G, const MeshArrays& M,
                            const int32_t* fixed, int nfixed, cudaStream_t s) {
@@ -2772,9 +2781,10 @@ void launch_inverse_ids(int n, const int32_t* id, int32_t* inv, cudaStream_t s) 
 }
 void launch_download(int count, int mode, const int32_t* inv, int id_lo, double* dst, float* const* src,
                      cudaStream_t s) {
+    const int nb = conv_blocks(count, kConvThreads);
     if (count > 0)
-        k_download<<<conv_grid(count, conv_groups(mode)), kConvThreads, 0, s>>>(count, mode, inv, id_lo, dst,
-                                                                                field_ptrs(src, mode));
+        k_download<<<conv_columns(mode) * nb, kConvThreads, 0, s>>>(count, nb, mode, inv, id_lo, dst,
+                                                                    field_set(src, mode));
 }
 void launch_init_particles(int n, const PArrays& cur, const uint8_t* mat, int has_fp, int track_fp, cudaStream_t s,
                            int id0, int fixed_mat, const int32_t* map) {
