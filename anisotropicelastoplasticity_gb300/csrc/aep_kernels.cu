@@ -2380,7 +2380,7 @@ __global__ void __launch_bounds__(kConvThreads) k_download_particles(int n, int 
         field(dst.Fp, P.Fp[0], 0) || field(dst.vol, P.vol, 1) || field(dst.plastic, P.plastic, 1);
 }
 
-// F_E (or F_P) into a device array from the slots' order: a warp's 32 matrices go through
+// F_P into a device array from the slots' order: a warp's 32 matrices go through
 // shared memory and leave as 72-byte pieces, nine lanes each
 __global__ void __launch_bounds__(kConvThreads) k_download_F_slots(int slots, int n, double* __restrict__ dst,
                                                                    FieldSet F, const int32_t* __restrict__ id) {
@@ -2503,40 +2503,6 @@ __global__ void k_init_particles(int n, PArrays cur, const uint8_t* __restrict__
     cur.mat[p] = (uint8_t)mat;
     if (!has_fp && track_fp)
         for (int k = 0; k < 9; ++k) cur.Fp[k][p] = (k % 4 == 0) ? 1.0f : 0.0f;
-}
-
-// snow particles carry J_P = det F_P in `plastic` when F_P is not tracked
-__global__ void k_snow_jp(int n, PArrays cur, const double* __restrict__ Fp, const int32_t* __restrict__ map) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n) return;
-    const int p = map ? map[q] : q;
-    if (cur.mat[p] != kSnow) return;
-    double A[9];
-    for (int a = 0; a < 3; ++a)
-        for (int b = 0; b < 3; ++b) A[3 * a + b] = Fp ? Fp[9l * q + a + 3 * b] : (a == b ? 1.0 : 0.0);
-    cur.plastic[p] = (float)mat_det(A);
-}
-
-// upload validation: largest mass (bit pattern of a non-negative double is monotonic),
-// bad masses (negative, NaN, inf) and unknown material tags; out = {max bits, bad}
-__global__ void k_check_upload(int n, const double* __restrict__ m, const uint8_t* __restrict__ mat,
-                               unsigned long long* out) {
-    unsigned long long mx = 0ull, bad = 0ull;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const double v = m[i];
-        if (!(v >= 0.0) || !isfinite(v)) bad = 1ull;
-        else if (v > 0.0) mx = max(mx, (unsigned long long)__double_as_longlong(v));
-        if (mat && mat[i] > kSand) bad = 1ull;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (mx) atomicMax(out, mx);
-        if (bad) atomicOr(out + 1, bad);
-    }
 }
 
 // inverse of the id map of the current order: inv[id[j]] = j
@@ -2737,7 +2703,9 @@ void launch_download_records(int slots, int n, const DownloadDst& dst, const PAr
     float4* const r = static_cast<float4*>(rec);
     k_slots_to_items<<<blocks_for(slots, kRecThreads), kRecThreads, 0, s>>>(slots, 0, n, P, r);
     k_unpack_items<<<blocks_for(n, kRecThreads), kRecThreads, 0, s>>>(n, r, dst);
-    if (dst.Fp) launch_download_F_slots(slots, n, dst.Fp, P.Fp, P.id, s);
+    if (dst.Fp)
+        k_download_F_slots<<<blocks_for(slots, kConvThreads), kConvThreads, 0, s>>>(slots, n, dst.Fp, field_set(P.Fp, 2),
+                                                                                    P.id);
 }
 void launch_upload_mesh(int slots, int id0, const MeshFields<const double>& m, const PArrays& P, void* rec,
                         cudaStream_t s) {
@@ -2756,10 +2724,6 @@ void launch_download_particles(int n, const DownloadDst& dst, const PArrays& P, 
                         (dst.Fe ? 9 : 0) + (dst.Fp ? 9 : 0);
     if (n > 0 && columns > 0) k_download_particles<<<columns * nb, kConvThreads, 0, s>>>(n, nb, dst, P, inv);
 }
-void launch_download_F_slots(int slots, int n, double* dst, float* const* F, const int32_t* id, cudaStream_t s) {
-    if (slots > 0)
-        k_download_F_slots<<<blocks_for(slots, kConvThreads), kConvThreads, 0, s>>>(slots, n, dst, field_set(F, 2), id);
-}
 void launch_fixed_vertices(const KParams& P, const PArrays& cur, const GArrays& G, const MeshArrays& M,
                            const int32_t* fixed, int nfixed, cudaStream_t s) {
     const long threads = (long)nfixed * 64 * 27;
@@ -2772,9 +2736,6 @@ void launch_query_weights(const KParams& P, const PArrays& cur, const int32_t* i
                           int64_t* nodes, double* w, double* g, cudaStream_t s) {
     const long threads = (long)count * 64;
     if (threads > 0) k_query_weights<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(P, cur, inv, ids, count, nodes, w, g);
-}
-void launch_check_upload(int n, const double* m, const uint8_t* mat, unsigned long long* out, cudaStream_t s) {
-    if (n > 0) k_check_upload<<<std::min(1024, blocks_for(n, 256)), 256, 0, s>>>(n, m, mat, out);
 }
 void launch_inverse_ids(int n, const int32_t* id, int32_t* inv, cudaStream_t s) {
     if (n > 0) k_inverse_ids<<<blocks_for(n, 256), 256, 0, s>>>(n, id, inv);
@@ -2789,9 +2750,6 @@ void launch_download(int count, int mode, const int32_t* inv, int id_lo, double*
 void launch_init_particles(int n, const PArrays& cur, const uint8_t* mat, int has_fp, int track_fp, cudaStream_t s,
                            int id0, int fixed_mat, const int32_t* map) {
     if (n > 0) k_init_particles<<<blocks_for(n, 256), 256, 0, s>>>(n, cur, mat, has_fp, track_fp, id0, fixed_mat, map);
-}
-void launch_snow_jp(int n, const PArrays& cur, const double* Fp, cudaStream_t s, const int32_t* map) {
-    if (n > 0) k_snow_jp<<<blocks_for(n, 256), 256, 0, s>>>(n, cur, Fp, map);
 }
 void launch_grid_dense(const KParams& P, const GArrays& G, double* mass, double* vel, double* vbf, int grid_blocks,
                        cudaStream_t s) {

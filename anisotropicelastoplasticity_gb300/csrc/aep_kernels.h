@@ -55,19 +55,16 @@ void launch_upload_particles(int n, const UploadSrc& src, const PArrays& P, cons
 void launch_upload_records(int slots, int n, const UploadSrc& src, const PArrays& P, int track_fp, void* rec,
                            unsigned long long* check, cudaStream_t s);
 void launch_download_records(int slots, int n, const DownloadDst& dst, const PArrays& P, void* rec, cudaStream_t s);
-void launch_download_F_slots(int slots, int n, double* dst, float* const* F, const int32_t* id, cudaStream_t s);
 void launch_download_particles(int n, const DownloadDst& dst, const PArrays& P, const int32_t* inv, cudaStream_t s);
 void launch_fixed_vertices(const KParams& P, const PArrays& cur, const GArrays& G, const MeshArrays& M,
                            const int32_t* fixed, int nfixed, cudaStream_t s);
 void launch_solve_dt(SolveState* S, int phase, const DevStats* st, unsigned long long* seen, cudaStream_t s);
 void launch_query_weights(const KParams& P, const PArrays& cur, const int32_t* inv, const int64_t* ids, int count,
                           int64_t* nodes, double* w, double* g, cudaStream_t s);
-void launch_check_upload(int n, const double* m, const uint8_t* mat, unsigned long long* out, cudaStream_t s);
 void launch_download(int count, int mode, const int32_t* inv, int id_lo, double* dst, float* const* src,
                      cudaStream_t s);
 void launch_init_particles(int n, const PArrays& cur, const uint8_t* mat, int has_fp, int track_fp,
                            cudaStream_t s, int id0 = 0, int fixed_mat = -1, const int32_t* map = nullptr);
-void launch_snow_jp(int n, const PArrays& cur, const double* Fp, cudaStream_t s, const int32_t* map = nullptr);
 void launch_grid_dense(const KParams& P, const GArrays& G, double* mass, double* vel, double* vbf,
                        int grid_blocks, cudaStream_t s);
 

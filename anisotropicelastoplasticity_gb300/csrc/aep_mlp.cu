@@ -77,8 +77,7 @@ __device__ __forceinline__ void strip_mma(float (&c)[4][4], const bf16* A, int a
     }
 }
 
-// 87,136 bytes: two blocks fit on an SM.  Rows of 24 and 72 halves: the eight rows of an
-// ldmatrix lie on distinct banks.
+// Rows of 24 and 72 halves: the eight rows of an ldmatrix lie on distinct banks.
 struct __align__(16) TrainSmem {
     bf16 W1[64 * kStrideIn], W2[64 * kStrideH], W3[64 * kStrideH], W4[8 * kStrideH];  // W^T
     bf16 X[kTrainRows * kStrideIn];
@@ -90,6 +89,7 @@ struct __align__(16) TrainSmem {
     float g1[64 * 17];  // W1's gradient, before its hi and lo columns are added
     float wloss[kTrainWarps];
 };
+static_assert(sizeof(TrainSmem) == 88256, "two blocks on an SM of 227 KB");
 
 __device__ __forceinline__ float dsilu(float z) {
     const float s = __frcp_rn(1.0f + __expf(-z));
