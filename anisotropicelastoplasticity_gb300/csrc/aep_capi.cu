@@ -411,9 +411,8 @@ aep_status download(aep_solver* s, double* dst, int count, int mode, float* cons
 }
 
 // Which exchanges with device memory go by way of records.  A record costs 27 x 4 + 2 x 128
-// bytes whatever is asked for and one kernel more; a value read on its own costs a 32-byte
-// sector.  Measured, us of a call by records / in the caller's order:
-//   readback of 26 values: 23.5 / 21.7 for 8,192 items, 24.5 / 24.8 for 32,768, 26.5 / 28.7
+// bytes whatever is asked for, a value read on its own a 32-byte sector.  Measured, us of a call by records / in the caller's order:
+//   readback of 26 values: 23.5 / 21 for 8,192 items, 24.4 / 24.5 for 32,768, 26.5 / 28.6
 //     for 65,536, 126 / 165 for 1,000,000; with F_P (35 values), a kernel more: 30.8 / 26.9
 //     for 32,768, 38 / 38 for 100,003, 59 / 70 for 262,144
 //   readback of 12 values: 19 / 17 for 8,192, 100 / 85 for 1,000,000; of 15: 106 / 103; of
@@ -426,7 +425,7 @@ constexpr int64_t kRecordReadback = 32768, kRecordReadbackFp = 100000, kRecordUp
 // Mesh state by way of records: two kernels over every item, against one for each array given
 // (and one for the inverse of the ids).  All seven arrays: 24 / 46 us for 4,225 vertices (their
 // triangles are twice as many), 37 / 58 for 66,049, 98 / 119 for 263,169, 332 / 337 for
-// 1,050,625; three of the vertices': 22 / 26 for 16,641, 31 / 28 for 66,049, 78 / 39 for
+// 1,050,625; three of the vertices': 21 / 26 for 4,225, 31 / 28 for 66,049, 78 / 39 for
 // 263,169; five of both: 23 / 27, 32 / 33 and 88 / 75.
 constexpr int kRecordMeshArrays = 3, kRecordMeshArraysLarge = 6;
 constexpr int64_t kRecordMeshLarge = 150000;  // items
@@ -436,14 +435,14 @@ template <typename T>
 bool mesh_by_records(const MeshFields<T>& m) {
     T* const all[] = {m.xv, m.vv, m.Bv, m.xe, m.ve, m.Be, m.d};
     int arrays = 0;
+    for (T* a : all) arrays += a != nullptr;
+    if (arrays < ((int64_t)m.nv + m.nf < kRecordMeshLarge ? kRecordMeshArrays : kRecordMeshArraysLarge)) return false;
     for (T* a : all) {
-        if (!a) continue;
         bool on_device = false;
         device_alias(a, &on_device);
-        if (!on_device) return false;
-        ++arrays;
+        if (a && !on_device) return false;
     }
-    return arrays >= ((int64_t)m.nv + m.nf < kRecordMeshLarge ? kRecordMeshArrays : kRecordMeshArraysLarge);
+    return true;
 }
 
 aep_status check_overflow(aep_solver* s) {
@@ -683,6 +682,13 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
     if (!keep_order) s->n = n;
     s->np = n;
     PArrays& P = s->P[s->cur];
+    const bool records = keep_order && n >= kRecordUpload;  // where every array is device memory
+    auto slots = [&]() {  // perm[id] = slot, over every item: ids 0..n-1 first
+        launch_inverse_ids((int)s->n, P.id, s->perm, s->stream);
+        return cudaGetLastError();
+    };
+    // first, to run while the arrays are looked up
+    if (keep_order && !records) CK(slots());
     // Arrays in page-locked host or device memory are read by the conversion
     // kernels directly; pageable ones are staged first (doubles): x 0, v 3n, B 6n,
     // Fe 15n, Fp 24n, m 33n, vol 34n, plastic 35n, material bytes at 36n.
@@ -709,18 +715,14 @@ aep_status aep_set_particles(aep_solver* s, int64_t n, const double* x, const do
     // the whole upload and its validation (bad masses, unknown tags, largest mass)
     // in one launch, read back with the final synchronisation
     CK(cudaMemsetAsync(s->check, 0, 2 * sizeof(unsigned long long), s->stream));
-    if (keep_order && all_on_device && n >= kRecordUpload) {
+    if (records && all_on_device) {
         // by way of records, in the staging buffer (16 of its 37 doubles per item; unused here)
         launch_upload_records((int)s->n, (int)n, src, P, s->prm.track_plastic_F, s->staging, s->check, s->stream);
     } else {
         // host memory is read in its own order, whole lines over the link
-        const int32_t* map = nullptr;
-        if (keep_order) {
-            launch_inverse_ids((int)s->n, P.id, s->perm, s->stream);  // over every item: ids 0..n-1 first
-            CKLAUNCH();
-            map = s->perm;
-        }
-        launch_upload_particles((int)n, src, P, map, s->prm.track_plastic_F, s->check, s->stream);
+        if (records) CK(slots());
+        launch_upload_particles((int)n, src, P, keep_order ? s->perm : nullptr, s->prm.track_plastic_F, s->check,
+                                s->stream);
     }
     CKLAUNCH();
     unsigned long long* chk = s->check_host;
@@ -1150,8 +1152,8 @@ aep_status aep_solve(aep_solver* s, double cfl, double maxt, double alpha) {
     // certain to follow: no callback may end the solve, t, which only moves at the end of a
     // frame, cannot move in the step in flight (Dt <= CFL / 300), and that step is past its
     // normalisation without an overflow.  Waiting for the end of every step before the launch
-    // of the next left the device idle between them (snow: 77 -> 73 us a step at 512
-    // particles, 73 -> 70 at 32,768, 105 -> 98 at 131,072, 241 -> 237 at 524,288).
+    // of the next left the device idle between them (snow: 77.5 -> 74 us a step at 512
+    // particles, 73 -> 70 at 32,768, 105 -> 100 at 131,072, 242 -> 238 at 524,288).
     double t = 0.0, inner = 0.0;  // after the last step read
     int64_t launched = 0, read = 0;
     // whether step i (from 1) went through its normalisation without an overflow; waits until
@@ -1496,22 +1498,26 @@ aep_status aep_get_particles(aep_solver* s, int64_t n, double* x, double* v, dou
     double* const req[7] = {x, v, B, Fe, Fp, vol, plastic};
     const size_t cnt[7] = {3, 3, 9, 9, 9, 1, 1}, off[7] = {0, 3, 6, 15, 24, 33, 34};
     double* dev[7] = {};
-    bool all_on_device = true;
     int values = 0;  // of the record, per item
+    for (int f = 0; f < 7; ++f) values += req[f] && f != 4 ? (int)cnt[f] : 0;
+    // where every array is device memory
+    const bool records = values >= kRecordValues && np >= (Fp ? kRecordReadbackFp : kRecordReadback);
+    // first, to run while the arrays are looked up (2,000 particles 20.7 -> 19.6 us)
+    if (!records && (st = prepare_download(s))) return st;
+    bool all_on_device = true;
     for (int f = 0; f < 7; ++f)
         if (req[f]) {
             bool on_device = false;
             double* a = static_cast<double*>(const_cast<void*>(device_alias(req[f], &on_device)));
             dev[f] = a ? a : s->staging + off[f] * N;
             all_on_device &= on_device;
-            values += f == 4 ? 0 : (int)cnt[f];
         }
     const DownloadDst dst{dev[0], dev[1], dev[2], dev[3], dev[4], dev[5], dev[6]};
-    if (all_on_device && values >= kRecordValues && np >= (Fp ? kRecordReadbackFp : kRecordReadback)) {
+    if (records && all_on_device) {
         launch_download_records((int)s->n, (int)np, dst, P, s->staging, s->stream);
         CKLAUNCH();
     } else {
-        if ((st = prepare_download(s))) return st;
+        if (records && (st = prepare_download(s))) return st;
         launch_download_particles((int)np, dst, P, s->inv, s->stream);
         CKLAUNCH();
         for (int f = 0; f < 7; ++f)
