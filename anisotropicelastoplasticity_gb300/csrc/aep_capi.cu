@@ -411,7 +411,8 @@ aep_status download(aep_solver* s, double* dst, int count, int mode, float* cons
 }
 
 // Which exchanges with device memory go by way of records.  A record costs 27 x 4 + 2 x 128
-// bytes whatever is asked for, a value read on its own a 32-byte sector.  Measured, us of a call by records / in the caller's order:
+// bytes whatever is asked for, a value read on its own a 32-byte sector.  Measured, us of a
+// call by records / in the caller's order:
 //   readback of 26 values: 23.5 / 21 for 8,192 items, 24.4 / 24.5 for 32,768, 26.5 / 28.6
 //     for 65,536, 126 / 165 for 1,000,000; with F_P (35 values), a kernel more: 30.8 / 26.9
 //     for 32,768, 38 / 38 for 100,003, 59 / 70 for 262,144
